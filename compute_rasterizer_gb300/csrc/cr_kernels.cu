@@ -270,7 +270,7 @@ __device__ __forceinline__ void decode_point(const uint4& w4, const uint4& w8, c
 }
 
 // LC: 2 = 10 bit (levels 2-4), 1 = 20 bit (level 1), 0 = 30 bit (level 0).
-// Points [first, first + count) are read as 128-bit vectors starting at the
+// Vectors [vb, ve) of the points [first, first + count) are read as 128-bit vectors starting at the
 // aligned word below `first`; lanes mask the words outside the range.  The
 // next vector is loaded before the current one is processed.  PAIRS (full
 // 10-bit batches that the cull flagged w-safe): points are decoded and
@@ -279,7 +279,7 @@ template <int MODE, int PAYLOAD, int BLOCK, int LC, bool FULL = false, bool PAIR
           bool LIT = false>
 __device__ __forceinline__ void run_points(const BatchedLaunch& bl, unsigned long long* zc,
                                            const BatchCtx& c, const PairParams& pp, int64_t first,
-                                           int32_t count, bool l0_x12) {
+                                           int32_t count, bool l0_x12, int vb, int ve) {
     static_assert(!PAIRS || (FULL && LC == 2), "pairs decode full 10-bit batches");
     PairCol3 pf{};
     if constexpr (PAIRS) pf = PairCol3{f2_pack(c.T12, c.T12), f2_pack(c.T13, c.T13), f2_pack(c.T15, c.T15)};
@@ -294,7 +294,8 @@ __device__ __forceinline__ void run_points(const BatchedLaunch& bl, unsigned lon
     // addressing is the same as here.  Only the raster reads this way (HQS
     // passes walk their batches with stride 128, hqs/depth.cs:270-276).
     const bool uvec4 = MODE == kModeRaster && !FULL && head != 0 && (bl.quirks & CR_QUIRK_UVEC4_BASE) != 0;
-    const int nv = uvec4 ? min((head + count + 3) >> 2, kPointsPerBatch / 4) : (head + count + 3) >> 2;
+    const int nv = min(ve, uvec4 ? min((head + count + 3) >> 2, kPointsPerBatch / 4)
+                                 : (head + count + 3) >> 2);
     const uint32_t index0 = (uint32_t)(first - head);  // global index of word 0 of vector v0
     const uint4* lo4 = reinterpret_cast<const uint4*>(bl.lo) + v0;
     const uint4* md4 = reinterpret_cast<const uint4*>(bl.md) + v0;
@@ -304,13 +305,13 @@ __device__ __forceinline__ void run_points(const BatchedLaunch& bl, unsigned lon
     uint4 n4 = zero, n8 = zero, n12 = zero, ncol = zero;
     PairBatch pb{};
     if constexpr (PAIRS) pb = pair_batch(c);
-    if ((int)threadIdx.x < nv) {
-        n4 = ld_stream(lo4 + threadIdx.x);
-        if (LC <= 1) n8 = ld_stream(md4 + threadIdx.x);
-        if (LC == 0) n12 = ld_stream(hi4 + threadIdx.x);
-        if (kNeedColor) ncol = ld_stream(co4 + threadIdx.x);
+    if (vb + (int)threadIdx.x < nv) {
+        n4 = ld_stream(lo4 + vb + threadIdx.x);
+        if (LC <= 1) n8 = ld_stream(md4 + vb + threadIdx.x);
+        if (LC == 0) n12 = ld_stream(hi4 + vb + threadIdx.x);
+        if (kNeedColor) ncol = ld_stream(co4 + vb + threadIdx.x);
     }
-    for (int base = 0; base < nv; base += BLOCK) {
+    for (int base = vb; base < nv; base += BLOCK) {
         const int v = base + (int)threadIdx.x;
         const uint4 w4 = n4, w8 = n8, w12 = n12, col = ncol;
         const int vn = v + BLOCK;
@@ -414,6 +415,43 @@ __device__ __forceinline__ void run_points(const BatchedLaunch& bl, unsigned lon
 template <int MODE, int BLOCK, int LIST, bool UNCAPPED = false>
 constexpr int kMinBlocks = MODE == kModeHqsColor && LIST == 0 && !UNCAPPED ? 1280 / BLOCK : 0;
 
+// How a launch hands out `nitems` list items to its CTAs: the first `whole`
+// items as one unit each, every later item as `parts` units of `part_vectors`
+// vectors.
+//
+// A CTA walks a whole batch in 20 serial steps of 512 points, about 16 us alone
+// and 30 us on a full SM, so a frame with few items left most SMs idle and
+// every frame ended in a wave of whole batches.  The last item per CTA goes out
+// in fifths (4 steps), and in tenths or single steps while there would be fewer
+// than two parts per CTA.  Items before those stay whole: a unit costs about a
+// step (cursor, record and first vectors, one after the other), and cutting
+// every batch measured 3-9 % slower on the 100M-point flight.  Frames, whole
+// batches -> parts: 50k points 32.9 -> 22.6 us, octree of 2M 54.2 -> 46.2,
+// 15M points in 24 files 121 -> 85, 100M-point flight (5 poses) 930 -> 897; a
+// billion points 1572 -> 1576 (its last wave is small beside its length).
+struct WorkSplit {
+    uint32_t whole, parts, units;
+    int part_vectors;
+};
+constexpr int kAllVectors = 1 << 30;
+
+template <int BLOCK>
+__device__ __forceinline__ WorkSplit split_work(uint32_t nitems, uint32_t ctas, int node_slices) {
+    // parts are whole steps of the CTA: 2,560 vectors of a batch (640 of a
+    // node slice) are `steps` steps of BLOCK vectors
+    const uint32_t steps = (node_slices ? kNodeSlice : kPointsPerBatch) / (4 * BLOCK);
+    uint32_t parts = steps % 5 == 0 ? 5 : 1;
+    if (nitems * parts < 2 * ctas) parts = steps % 10 == 0 ? 10 : steps;
+    if (nitems * parts < 2 * ctas) parts = steps;
+    WorkSplit w;
+    w.parts = parts > 0 ? parts : 1;
+    w.part_vectors = (int)(max(steps / w.parts, 1u) * BLOCK);
+    const uint32_t split = min(nitems, ctas);
+    w.whole = nitems - split;
+    w.units = w.whole + split * w.parts;
+    return w;
+}
+
 // LIST 0: the 10-bit items (front of the list region), LIST 1: the 20/30-bit
 // items (back of the region).  Each list runs in its own instance, so the
 // common 10-bit instance carries no wider decode state (fewer registers).
@@ -435,16 +473,27 @@ __global__ void __launch_bounds__(BLOCK, (kMinBlocks<MODE, BLOCK, LIST, MANY && 
                                                : (MODE == kModeHqsColor ? kCursor3 : kCursor2));
     const uint32_t nitems =
         *reinterpret_cast<volatile uint32_t*>(bl.scratch + (LIST == 0 ? kItemCount : kItemCount2));
-    if (nitems != 0) {
+    const WorkSplit ws = split_work<BLOCK>(nitems, gridDim.x, bl.node_slices);
+    if (blockIdx.x < ws.units) {
         if (MODE != kModeHqsColor)
             for (int i = threadIdx.x; i < kZCacheSlots; i += BLOCK) s_zc[i] = 0xFFFFFFFFull;
-        if (threadIdx.x == 0) s_item[0] = atomicAdd(cursor, 1u);
+        // the first unit is the CTA's own number; the cursor hands out the rest
+        if (threadIdx.x == 0) s_item[0] = blockIdx.x;
         __syncthreads();
         int buf = 0;
         while (true) {
-            const uint32_t wi = s_item[buf];
-            if (wi >= nitems) break;
-            if (threadIdx.x == 0) s_item[buf ^ 1] = atomicAdd(cursor, 1u);
+            const uint32_t unit = s_item[buf];
+            if (unit >= ws.units) break;
+            if (threadIdx.x == 0) s_item[buf ^ 1] = gridDim.x + atomicAdd(cursor, 1u);
+            uint32_t wi = unit, part = 0;
+            int vb = 0, ve = kAllVectors;
+            if (unit >= ws.whole) {
+                wi = ws.whole + (unit - ws.whole) / ws.parts;
+                part = (unit - ws.whole) % ws.parts;
+                vb = (int)part * ws.part_vectors;
+                // the last part of an unaligned batch takes its extra vector too
+                ve = part + 1 == ws.parts ? kAllVectors : vb + ws.part_vectors;
+            }
             const uint32_t item =
                 bl.scratch[kScratchHead + (LIST == 0 ? (int64_t)wi : bl.list_cap - 1 - (int64_t)wi)];
             const uint32_t b = item & (bl.node_slices ? kItemNodeMask : kItemBatchMask);
@@ -489,13 +538,13 @@ __global__ void __launch_bounds__(BLOCK, (kMinBlocks<MODE, BLOCK, LIST, MANY && 
                 (count == kPointsPerBatch ||
                  (kNodeSlice % (4 * BLOCK) == 0 && bl.node_slices && count == kNodeSlice)) &&
                 (first & 3) == 0 && pair_batch_exact(c))
-                run_points<MODE, PAYLOAD, BLOCK, 2, true, true, LIT>(bl, s_zc, c, pp, first, count, l0_x12);
+                run_points<MODE, PAYLOAD, BLOCK, 2, true, true, LIT>(bl, s_zc, c, pp, first, count, l0_x12, vb, ve);
             else if (LIST == 0)
-                run_points<MODE, PAYLOAD, BLOCK, 2, false, false, LIT>(bl, s_zc, c, pp, first, count, l0_x12);
+                run_points<MODE, PAYLOAD, BLOCK, 2, false, false, LIT>(bl, s_zc, c, pp, first, count, l0_x12, vb, ve);
             else if (level == 1)
-                run_points<MODE, PAYLOAD, BLOCK, 1, false, false, LIT>(bl, s_zc, c, pp, first, count, l0_x12);
+                run_points<MODE, PAYLOAD, BLOCK, 1, false, false, LIT>(bl, s_zc, c, pp, first, count, l0_x12, vb, ve);
             else
-                run_points<MODE, PAYLOAD, BLOCK, 0, false, false, LIT>(bl, s_zc, c, pp, first, count, l0_x12);
+                run_points<MODE, PAYLOAD, BLOCK, 0, false, false, LIT>(bl, s_zc, c, pp, first, count, l0_x12, vb, ve);
             __syncthreads();
             buf ^= 1;
         }

@@ -1,0 +1,54 @@
+"""The unit split of the batched kernels (whole batches first, the last item
+per CTA in parts): item counts around every switch of the rule, against the
+oracle, bit for bit."""
+import numpy as np
+import pytest
+
+from compute_rasterizer_gb300 import _lib as L
+from helpers import QUIRKS, cameras, encoded, first_diff, gpu_raw, oracle_frame
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+BATCHES = 310
+
+
+@pytest.fixture(scope="module")
+def cloud_310(ctx):
+    n = (BATCHES - 1) * L.POINTS_PER_BATCH + 6_001  # the last batch is partial
+    cl = encoded(n=n, extent=800.0, seed=23)
+    cloud = ctx.cloud_from_arrays(cl["batches"], cl["lo"], cl["md"], cl["hi"], cl["rgba"],
+                                  cl["box_min"])
+    yield cl, cloud
+    cloud.close()
+
+
+# With one CTA per SM (152): 20 parts below 31 items, 10 below 61, 5 from there,
+# whole items from 153; 153 with two CTAs per SM is again below two parts a CTA.
+@pytest.mark.parametrize("block", [128, 256, 512])
+@pytest.mark.parametrize("items,ctas", [(1, 1), (30, 1), (31, 1), (60, 1), (61, 1), (152, 1),
+                                        (153, 1), (153, 2), (310, 1)])
+def test_item_counts(ctx, cloud_310, items, ctas, block):
+    cl, cloud = cloud_310
+    points = min(cl["n"], items * L.POINTS_PER_BATCH)
+    cloud.set_loaded(points, items)
+    cam = cameras(cl)["far"]
+    try:
+        fb, _ = gpu_raw(ctx, cloud, cam, L.METHOD_LOOP_LAS, L.PAYLOAD_INDEX, culling=0,
+                        block_threads=block, ctas_per_sm=ctas)
+        fr = oracle_frame(cam, cl["box_min"][None], QUIRKS[L.METHOD_LOOP_LAS], culling=0)
+        want = O.raster_batched(fr, cl["batches"][:items], points, cl["lo"], cl["md"], cl["hi"],
+                                cl["rgba"])
+        got = fb.read(L.FB_WORDS)
+        assert np.array_equal(got, want), first_diff(got, want)
+        fb.close()
+        fb, _ = gpu_raw(ctx, cloud, cam, L.METHOD_LOOP_LAS_HQS, culling=0, block_threads=block,
+                        ctas_per_sm=ctas)
+        fr = oracle_frame(cam, cl["box_min"][None], QUIRKS[L.METHOD_LOOP_LAS_HQS], culling=0)
+        depth, accum, _ = O.hqs(fr, cl["batches"][:items], points, cl["lo"], cl["md"], cl["hi"],
+                                cl["rgba"])
+        assert np.array_equal(fb.read(L.FB_DEPTH), depth)
+        assert np.array_equal(fb.read(L.FB_ACCUM), accum)
+        fb.close()
+    finally:
+        cloud.set_loaded()
