@@ -924,8 +924,9 @@ cr_status cr_last_frame_stats(cr_ctx* ctx, const cr_cloud* cloud, const cr_rende
     for (uint32_t it : items) {
         const uint32_t b = it & (ctx->last_node_slices ? kItemNodeMask : kItemBatchMask);
         const int64_t slice = ctx->last_node_slices ? (int64_t)((it >> kItemSliceShift) & 31u) : 0;
-        const int level = (int)(it >> 29);
-        if (b >= recs.size() || level > 4) continue;
+        const int code = (int)(it >> 29);
+        const int level = code > 4 ? code - kLevelInside : code;
+        if (b >= recs.size()) continue;
         int64_t n = recs[b].num_points;
         if (quirks & CR_QUIRK_NODE_LOOP) {  // compute_loop_nodes/render.cs:296-300
             const int64_t loop = std::min<int64_t>((n + 127) / 128, 500);

@@ -35,8 +35,8 @@ __device__ __forceinline__ float fsub(float a, float b) { return __fsub_rn(a, b)
 // on the conversion pipe, which the raster leaves mostly idle; it measured
 // faster than the two-instruction float trick on the issue-bound raster.
 __device__ __forceinline__ float small_u2f(uint32_t x) { return __uint2float_rn(x); }
-// int(f) by truncation, for the pixel coordinate (f >= 0 for every point
-// inside the view; the value of an outside point is never used).
+// int(f) by truncation, for the pixel coordinate of the scalar bodies (f >= 0 for
+// every point inside the view; the value of an outside point is never used).
 __device__ __forceinline__ int32_t small_f2i(float f) { return __float2int_rz(f); }
 
 __device__ __forceinline__ uint4 ld_stream(const uint4* p) {
@@ -110,6 +110,32 @@ __device__ __forceinline__ bool w_safe(const float* T, float mnx, float mny, flo
     }
     const float err = fmul(mag, 0x1p-16f);
     return fsub(lo, err) >= lo_bound && fadd(hi, err) <= hi_bound;
+}
+
+// Whether every point decoded from a batch that w_safe() passed projects inside
+// the view (|x / w| <= 1 and |y / w| <= 1): w - |x| and w - |y| are minima of
+// linear functions, so over the AABB they are least at corners.  The margin,
+// 2^-15 of the term sums of both rows, is far above the rounding of the two
+// rows (see w_safe) and of the quotient (2^-22 of w).
+__device__ __forceinline__ bool all_inside(const float* T, float mnx, float mny, float mnz, float mxx,
+                                           float mxy, float mxz) {
+    float slack = 0.0f, mag = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const float x = (k & 1) ? mxx : mnx, y = (k & 2) ? mxy : mny, z = (k & 4) ? mxz : mnz;
+        float p[3], m[3];
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+            const int c = r == 2 ? 3 : r;
+            p[r] = __fmaf_rn(T[8 + c], z, __fmaf_rn(T[4 + c], y, __fmaf_rn(T[c], x, T[12 + c])));
+            m[r] = fadd(fadd(fadd(fabsf(fmul(T[c], x)), fabsf(fmul(T[4 + c], y))),
+                             fabsf(fmul(T[8 + c], z))), fabsf(T[12 + c]));
+        }
+        const float s = fsub(p[2], fmaxf(fabsf(p[0]), fabsf(p[1])));
+        slack = k == 0 ? s : fminf(slack, s);
+        mag = fmaxf(mag, fadd(fadd(m[0], m[1]), m[2]));
+    }
+    return slack >= fmul(mag, 0x1p-15f);
 }
 
 // ---- per-batch math (render.cs:130-231), no contraction --------------------
@@ -221,14 +247,20 @@ struct BatchCtx {
 // framebuffer during the frame, so it is never below the word's final minimum
 // depth: a point deeper than the cached depth cannot win and is dropped
 // without touching global memory.  Entries are single 64-bit words, so a racing
-// writer replaces an entry but never tears one; the table starts empty (tag
-// 0xFFFFFFFF).
+// writer replaces an entry but never tears one; the table starts with depths
+// that reject nothing.
 constexpr int kZCacheBits = 11;
 constexpr int kZCacheSlots = 1 << kZCacheBits;
+constexpr unsigned long long kZCacheEmpty = ~0ull;  // a depth no point lies behind
 
 __device__ __forceinline__ uint32_t zslot(uint32_t tag) {
     return (tag * 2654435761u) >> (32 - kZCacheBits);
 }
+// The single-view bodies carry a pixel as pix + pixel_bias(W): the pair bodies
+// read int(f) as the bits of f + 2^23, which leaves this constant in ix + iy * W
+// (mod 2^32); it comes off only where a pixel is addressed.  Its low 24 bits are
+// zero, so the slot is the pixel's own.
+__device__ __forceinline__ uint32_t pixel_bias(int32_t W) { return 0x4B000000u * (1u + (uint32_t)W); }
 // Single-view slots: a CTA's batch covers a compact screen region, whose pixel
 // ids already differ in their low bits (measured faster than the hash there;
 // the multi-view tags, offset per view, keep the hash).
@@ -333,6 +365,7 @@ struct PairParams {
     uint64_t half, Wf, Hf;  // (0.5, 0.5), (W, W), (H, H)
     uint64_t bias;          // (-2^23, -2^23)
     uint64_t one, nhalf;    // (1, 1), (-0.5, -0.5)
+    uint64_t two23;         // (2^23, 2^23)
 };
 struct PairCol3 {
     uint64_t T12, T13, T15;  // the batch's file's translation column, as pairs
@@ -356,6 +389,11 @@ __device__ __forceinline__ uint64_t f2_pack(float lo, float hi) {
 __device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
     uint64_t d;
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t f2_add_rz(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("add.rz.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
 __device__ __forceinline__ void f2_unpack(uint64_t v, float& lo, float& hi) {
@@ -411,13 +449,14 @@ __device__ __forceinline__ uint64_t f2_add_scalar(uint64_t a, uint64_t b) {
     return f2_pack(fadd(a0, b0), fadd(a1, b1));
 }
 
-// A batch's 10-bit decode uniforms as pairs (per batch, in registers): the
-// steps sx, sy * 2^-10, sz * 2^-20 and the minimum corner (see project_pair10).
+// A batch's decode uniforms as pairs (per batch, in registers): the steps (at
+// 10 bit sx, sy * 2^-10, sz * 2^-20) and the minimum corner (see project_pair10).
 struct PairBatch {
     uint64_t sx, sy, sz, mnx, mny, mnz;
 };
+template <int LC>
 __device__ __forceinline__ PairBatch pair_batch(const BatchCtx& c) {
-    const float sy = fmul(c.sy, 0x1p-10f), sz = fmul(c.sz, 0x1p-20f);
+    const float sy = LC == 2 ? fmul(c.sy, 0x1p-10f) : c.sy, sz = LC == 2 ? fmul(c.sz, 0x1p-20f) : c.sz;
     return PairBatch{f2_pack(c.sx, c.sx), f2_pack(sy, sy), f2_pack(sz, sz),
                      f2_pack(c.mnx, c.mnx), f2_pack(c.mny, c.mny), f2_pack(c.mnz, c.mnz)};
 }
@@ -433,17 +472,19 @@ __device__ __forceinline__ bool pair_batch_exact(const BatchCtx& c) {
 // symmetric, and q * 0.5 + 0.5 is the same real value as NQ * -0.5 + 0.5, so
 // every result is the scalar path's.  LIT: a correctly rounded division per
 // component (f2_neg_div_rn) for the one reciprocal.
-template <bool LIT = false>
+template <bool LIT = false, bool INSIDE = false>
 __device__ __forceinline__ void project_pair_finish(uint64_t PX, uint64_t PY, uint64_t PW,
                                                     const PairParams& pp, int32_t W, bool ok[2],
-                                                    int32_t pix[2], uint32_t wbits[2]) {
+                                                    uint32_t pix[2], uint32_t wbits[2]) {
     // callers: w-safe batches only (every w in [2^-120, 2^120]; with LIT in
     // [2^-64, 2^64])
     const uint64_t NR = f2_neg_rcp_rn_normal(PW, pp.one);
     const uint64_t NQX = LIT ? f2_neg_div_rn(PX, PW, NR) : f2_mul(PX, NR);
     const uint64_t NQY = LIT ? f2_neg_div_rn(PY, PW, NR) : f2_mul(PY, NR);
-    const uint64_t FX = f2_mul(f2_fma(NQX, pp.nhalf, pp.half), pp.Wf);
-    const uint64_t FY = f2_mul(f2_fma(NQY, pp.nhalf, pp.half), pp.Hf);
+    // + 2^23 toward zero: the sum's bits are 0x4B000000 + int(f) for f in [0, 2^22),
+    // two conversions in one packed sum
+    const uint64_t FX = f2_add_rz(f2_mul(f2_fma(NQX, pp.nhalf, pp.half), pp.Wf), pp.two23);
+    const uint64_t FY = f2_add_rz(f2_mul(f2_fma(NQY, pp.nhalf, pp.half), pp.Hf), pp.two23);
     float pw[2], nqx[2], nqy[2], fx[2], fy[2];
     f2_unpack(PW, pw[0], pw[1]);
     f2_unpack(NQX, nqx[0], nqx[1]);
@@ -454,10 +495,41 @@ __device__ __forceinline__ void project_pair_finish(uint64_t PX, uint64_t PY, ui
     for (int k = 0; k < 2; k++) {
         // w >= 2^-120 for every point of a w-safe batch: render.cs:404's w > 0
         // holds, so only the x and y bounds are tested (HQS 3.334 -> 3.281 ms)
-        ok[k] = nqx[k] >= -1.0f && nqx[k] <= 1.0f && nqy[k] >= -1.0f && nqy[k] <= 1.0f;
-        pix[k] = small_f2i(fx[k]) + small_f2i(fy[k]) * W;
+        ok[k] = INSIDE || (fabsf(nqx[k]) <= 1.0f && fabsf(nqy[k]) <= 1.0f);
+        pix[k] = __float_as_uint(fx[k]) + __float_as_uint(fy[k]) * (uint32_t)W;
         wbits[k] = __float_as_uint(pw[k]);
     }
+}
+
+// Two points from their float coordinates in steps (XF, YF, ZF) through the
+// decode and project(), as pairs: the same operations in the same order,
+// element by element.
+template <bool LIT = false, bool INSIDE = false>
+__device__ __forceinline__ void project_pair(const PairParams& pp, const PairCol3& f,
+                                             const PairBatch& b, int32_t W, uint64_t XF, uint64_t YF,
+                                             uint64_t ZF, bool ok[2], uint32_t pix[2],
+                                             uint32_t wbits[2]) {
+    // project_clip: T0 T1 T3 T4 T5 T7 T8 T9 T11 are pp.T[0..8]
+    if (LIT) {
+        const uint64_t X = f2_add_scalar(f2_mul(XF, b.sx), b.mnx);
+        const uint64_t Y = f2_add_scalar(f2_mul(YF, b.sy), b.mny);
+        const uint64_t Z = f2_add_scalar(f2_mul(ZF, b.sz), b.mnz);
+        const uint64_t PX = f2_add(f2_add_scalar(f2_mul(pp.T[0], X), f2_mul(pp.T[3], Y)),
+                                   f2_add_scalar(f2_mul(pp.T[6], Z), f.T12));
+        const uint64_t PY = f2_add(f2_add_scalar(f2_mul(pp.T[1], X), f2_mul(pp.T[4], Y)),
+                                   f2_add_scalar(f2_mul(pp.T[7], Z), f.T13));
+        const uint64_t PW = f2_add(f2_add_scalar(f2_mul(pp.T[2], X), f2_mul(pp.T[5], Y)),
+                                   f2_add_scalar(f2_mul(pp.T[8], Z), f.T15));
+        project_pair_finish<true, INSIDE>(PX, PY, PW, pp, W, ok, pix, wbits);
+        return;
+    }
+    const uint64_t X = f2_fma(XF, b.sx, b.mnx);
+    const uint64_t Y = f2_fma(YF, b.sy, b.mny);
+    const uint64_t Z = f2_fma(ZF, b.sz, b.mnz);
+    const uint64_t PX = f2_fma(pp.T[6], Z, f2_fma(pp.T[3], Y, f2_fma(pp.T[0], X, f.T12)));
+    const uint64_t PY = f2_fma(pp.T[7], Z, f2_fma(pp.T[4], Y, f2_fma(pp.T[1], X, f.T13)));
+    const uint64_t PW = f2_fma(pp.T[8], Z, f2_fma(pp.T[5], Y, f2_fma(pp.T[2], X, f.T15)));
+    project_pair_finish<false, INSIDE>(PX, PY, PW, pp, W, ok, pix, wbits);
 }
 
 // Two 10-bit points (words a0, a1) through decode_point<2> and project(), as
@@ -477,10 +549,10 @@ __device__ __forceinline__ void project_pair_finish(uint64_t PX, uint64_t PY, ui
 // consumes it (the results came out 1 ulp off), while it leaves scalar sums
 // of a packed product's halves alone.  The outer sum of a row adds two sums
 // and runs as a pair.
-template <bool LIT = false>
+template <bool LIT = false, bool INSIDE = false>
 __device__ __forceinline__ void project_pair10(const PairParams& pp, const PairCol3& f,
                                                const PairBatch& b, int32_t W, uint32_t a0,
-                                               uint32_t a1, bool ok[2], int32_t pix[2],
+                                               uint32_t a1, bool ok[2], uint32_t pix[2],
                                                uint32_t wbits[2]) {
     const uint64_t XF = f2_add(f2_pack(__uint_as_float((a0 & 0x3FFu) | 0x4B000000u),
                                        __uint_as_float((a1 & 0x3FFu) | 0x4B000000u)), pp.bias);
@@ -488,27 +560,7 @@ __device__ __forceinline__ void project_pair10(const PairParams& pp, const PairC
                                        __uint_as_float((a1 & 0xFFC00u) | 0x4B000000u)), pp.bias);
     const uint64_t ZF =
         f2_pack(__uint2float_rn(a0 & 0x3FF00000u), __uint2float_rn(a1 & 0x3FF00000u));
-    // project_clip: T0 T1 T3 T4 T5 T7 T8 T9 T11 are pp.T[0..8]
-    if (LIT) {
-        const uint64_t X = f2_add_scalar(f2_mul(XF, b.sx), b.mnx);
-        const uint64_t Y = f2_add_scalar(f2_mul(YF, b.sy), b.mny);
-        const uint64_t Z = f2_add_scalar(f2_mul(ZF, b.sz), b.mnz);
-        const uint64_t PX = f2_add(f2_add_scalar(f2_mul(pp.T[0], X), f2_mul(pp.T[3], Y)),
-                                   f2_add_scalar(f2_mul(pp.T[6], Z), f.T12));
-        const uint64_t PY = f2_add(f2_add_scalar(f2_mul(pp.T[1], X), f2_mul(pp.T[4], Y)),
-                                   f2_add_scalar(f2_mul(pp.T[7], Z), f.T13));
-        const uint64_t PW = f2_add(f2_add_scalar(f2_mul(pp.T[2], X), f2_mul(pp.T[5], Y)),
-                                   f2_add_scalar(f2_mul(pp.T[8], Z), f.T15));
-        project_pair_finish<true>(PX, PY, PW, pp, W, ok, pix, wbits);
-        return;
-    }
-    const uint64_t X = f2_fma(XF, b.sx, b.mnx);
-    const uint64_t Y = f2_fma(YF, b.sy, b.mny);
-    const uint64_t Z = f2_fma(ZF, b.sz, b.mnz);
-    const uint64_t PX = f2_fma(pp.T[6], Z, f2_fma(pp.T[3], Y, f2_fma(pp.T[0], X, f.T12)));
-    const uint64_t PY = f2_fma(pp.T[7], Z, f2_fma(pp.T[4], Y, f2_fma(pp.T[1], X, f.T13)));
-    const uint64_t PW = f2_fma(pp.T[8], Z, f2_fma(pp.T[5], Y, f2_fma(pp.T[2], X, f.T15)));
-    project_pair_finish(PX, PY, PW, pp, W, ok, pix, wbits);
+    project_pair<LIT, INSIDE>(pp, f, b, W, XF, YF, ZF, ok, pix, wbits);
 }
 
 // Host side: the pair uniforms of a view (file 0's columns 0-2, which every
@@ -527,6 +579,7 @@ inline void fill_pair_params(const ViewParams& vp, PairParams* pp) {
     pp->Hf = dup((float)vp.H);
     pp->one = dup(1.0f);
     pp->nhalf = dup(-0.5f);
+    pp->two23 = dup(8388608.0f);
 }
 
 }  // namespace

@@ -39,6 +39,9 @@ constexpr int64_t kStreamPad = 64;
 constexpr uint32_t kItemBatchMask = 0x0FFFFFFFu;
 constexpr uint32_t kItemWSafe = 1u << 28;
 constexpr int64_t kMaxBatches = (int64_t)1 << 28;
+// Added to the level bits of a 10-bit item (levels 2-4) whose every point is
+// proven to project inside the view (all_inside): 5-7 are levels 2-4 of those.
+constexpr int kLevelInside = 3;
 // With node slicing (loop_nodes, whose nodes hold up to 64,512 points), a
 // node is handed out as items of kNodeSlice points: the slice in bits 23-27
 // and the node's record index below.  Slices far smaller than a node spread

@@ -13,14 +13,15 @@
 // Kernels
 //   k_cull      one thread per batch record: validation, frustum cull
 //               (render.cs:176-197), precision level (render.cs:199-231);
-//               w-safe flag (w_safe); appends (batch | flag | level << 29)
-//               to a work list.
+//               w-safe and inside flags (w_safe, all_inside); appends (batch |
+//               flag | level << 29) to a work list.
 //   k_batched   persistent CTAs pull work items; per batch the points are read
 //               with 128-bit streaming loads (4 consecutive points per lane,
 //               the loop_las2 `uvec4` scheme), decoded at 10/20/30 bit,
-//               projected (full 10-bit batches two points per packed
-//               instruction), tested against a per-CTA shared-memory z-cache,
-//               and the survivors issue 64-bit atomicMin (render.cs:399-432).
+//               projected (two points per packed instruction), merged per lane
+//               where they share a pixel, tested against a per-CTA
+//               shared-memory z-cache, and the survivors issue 64-bit atomicMin
+//               (render.cs:399-432).
 //               The same body runs the HQS depth pass (u32 atomicMin,
 //               hqs/depth.cs) and color pass (per-lane run sums; a lane's
 //               last run through __match_any_sync partitioned sums; two
@@ -109,8 +110,11 @@ __global__ void __launch_bounds__(256) k_cull(const __grid_constant__ ViewParams
                 const bool lit = (quirks & CR_QUIRK_LITERAL_ARITH) != 0;
                 const float wlo = lit ? 0x1p-64f : 0x1p-120f;
                 const float whi = lit ? 0x1p64f : 0x1p120f;
-                item = (uint32_t)b | ((uint32_t)level << 29) |
-                       (w_safe(f.T, mnx, mny, mnz, mxx, mxy, mxz, wlo, whi) ? kItemWSafe : 0u);
+                const bool safe = w_safe(f.T, mnx, mny, mnz, mxx, mxy, mxz, wlo, whi);
+                const bool inside =
+                    safe && level >= 2 && all_inside(f.T, mnx, mny, mnz, mxx, mxy, mxz);
+                item = (uint32_t)b | ((uint32_t)(inside ? level + kLevelInside : level) << 29) |
+                       (safe ? kItemWSafe : 0u);
                 if (node_slices) slices = (uint32_t)cr::node_slices(fp, count);
             }
         }
@@ -166,37 +170,35 @@ __global__ void __launch_bounds__(256) k_cull(const __grid_constant__ ViewParams
 
 // ---- batched raster / HQS body ---------------------------------------------
 
-// The raster and depth passes merge same-pixel candidates through the CTA's
-// z-cache rather than with __match_any_sync: a warp vote skips the atomic path
-// when no lane survives the cache test, and each surviving lane submits its
-// own 64-bit (or 32-bit) atomic min.  Measured on 1B points, a match-and-reduce
-// merge in front of the atomics made the frame 6-11% slower at every
-// threshold tried.
+// A candidate that survives the CTA's z-cache submits its own 64-bit (or
+// 32-bit) atomic min.  Lanes on one pixel are not merged with
+// __match_any_sync: in front of the atomics it made the 1B frame 6-11 % slower
+// at every threshold tried.  No warp vote skips the atomic path either: four
+// candidates in five warps have one (zoom 800M, color 1134 -> 1085 us without).
 template <>
 struct Emit<kModeRaster> {
     static __device__ __forceinline__ void run(const BatchedLaunch& bl, unsigned long long* zc,
-                                               bool ok, int32_t pix, uint32_t wbits,
-                                               uint32_t payload, uint32_t) {
-        const uint32_t slot = zslot_pixel((uint32_t)pix);
+                                               uint32_t bias, bool ok, uint32_t pix, uint32_t wbits,
+                                               uint32_t payload) {
+        const uint32_t slot = zslot_pixel(pix);
         // render.cs:423-424 early depth test, against the CTA's cache
-        const bool cand = ok && !zcache_rejects(zc, slot, (uint32_t)pix, wbits);
-        if (__any_sync(kFull, cand) && cand)
-            submit_min<unsigned long long>(reinterpret_cast<unsigned long long*>(bl.fb) + pix, zc,
-                                           slot, (uint32_t)pix,
-                                           ((unsigned long long)wbits << 32) | payload, wbits);
+        const bool cand = ok && !zcache_rejects(zc, slot, pix, wbits);
+        if (cand)
+            submit_min<unsigned long long>(reinterpret_cast<unsigned long long*>(bl.fb) + (pix - bias),
+                                           zc, slot, pix, ((unsigned long long)wbits << 32) | payload,
+                                           wbits);
     }
 };
 
 template <>
 struct Emit<kModeHqsDepth> {
     static __device__ __forceinline__ void run(const BatchedLaunch& bl, unsigned long long* zc,
-                                               bool ok, int32_t pix, uint32_t wbits, uint32_t,
+                                               uint32_t bias, bool ok, uint32_t pix, uint32_t wbits,
                                                uint32_t) {
-        const uint32_t slot = zslot_pixel((uint32_t)pix);
+        const uint32_t slot = zslot_pixel(pix);
         // hqs/depth.cs:375-379
-        const bool cand = ok && !zcache_rejects(zc, slot, (uint32_t)pix, wbits);
-        if (__any_sync(kFull, cand) && cand)
-            submit_min<uint32_t>(bl.depth + pix, zc, slot, (uint32_t)pix, wbits, wbits);
+        const bool cand = ok && !zcache_rejects(zc, slot, pix, wbits);
+        if (cand) submit_min<uint32_t>(bl.depth + (pix - bias), zc, slot, pix, wbits, wbits);
     }
 };
 
@@ -242,45 +244,99 @@ __device__ __forceinline__ float decode_axis(float X, float step, float mn) {
     return LIT ? fadd(fmul(X, step), mn) : __fmaf_rn(X, step, mn);
 }
 
-// Decodes point j of the lane's vector at level class LC (render.cs:333-397).
-template <int LC, bool LIT = false>
-__device__ __forceinline__ void decode_point(const uint4& w4, const uint4& w8, const uint4& w12, int j,
-                                             const BatchCtx& c, bool l0_x12, float& x, float& y,
-                                             float& z) {
+// The integer coordinates of point j of the lane's vector at level class LC
+// (render.cs:333-397).
+template <int LC>
+__device__ __forceinline__ void decode_fields(const uint4& w4, const uint4& w8, const uint4& w12, int j,
+                                              bool l0_x12, uint32_t q[3]) {
     const uint32_t a = u4get(w4, j);
     if (LC == 2) {
-        x = decode_axis<LIT>(small_u2f(a & 1023u), c.sx, c.mnx);
-        y = decode_axis<LIT>(small_u2f((a >> 10) & 1023u), c.sy, c.mny);
-        z = decode_axis<LIT>(small_u2f((a >> 20) & 1023u), c.sz, c.mnz);
-    } else {
-        const uint32_t b = u4get(w8, j);
-        uint32_t X = ((a & 1023u) << 20) | ((b & 1023u) << 10);
-        uint32_t Y = (((a >> 10) & 1023u) << 20) | (((b >> 10) & 1023u) << 10);
-        uint32_t Z = (((a >> 20) & 1023u) << 20) | (((b >> 20) & 1023u) << 10);
-        if (LC == 0) {
-            const uint32_t h = u4get(w12, j);
-            uint32_t x12 = h & 1023u, y12 = (h >> 10) & 1023u, z12 = (h >> 20) & 1023u;
-            if (l0_x12) { y12 = x12; z12 = x12; }
-            X |= x12; Y |= y12; Z |= z12;
-        }
-        x = decode_axis<LIT>(__uint2float_rn(X), c.sx, c.mnx);
-        y = decode_axis<LIT>(__uint2float_rn(Y), c.sy, c.mny);
-        z = decode_axis<LIT>(__uint2float_rn(Z), c.sz, c.mnz);
+        q[0] = a & 1023u;
+        q[1] = (a >> 10) & 1023u;
+        q[2] = (a >> 20) & 1023u;
+        return;
+    }
+    const uint32_t b = u4get(w8, j);
+    q[0] = ((a & 1023u) << 20) | ((b & 1023u) << 10);
+    q[1] = (((a >> 10) & 1023u) << 20) | (((b >> 10) & 1023u) << 10);
+    q[2] = (((a >> 20) & 1023u) << 20) | (((b >> 20) & 1023u) << 10);
+    if (LC == 0) {
+        const uint32_t h = u4get(w12, j);
+        uint32_t x12 = h & 1023u, y12 = (h >> 10) & 1023u, z12 = (h >> 20) & 1023u;
+        if (l0_x12) { y12 = x12; z12 = x12; }
+        q[0] |= x12; q[1] |= y12; q[2] |= z12;
     }
 }
 
+// How a unit's points are projected.  Every body computes the same words.
+//
+// kBodyPair takes any w-safe unit: words outside the batch decode inside its
+// AABB like any others, so only their results are masked.  Whole aligned batches
+// alone went in pairs before, and batches that start at any word (every file of
+// a mosaic but the first) or decode at 20/30 bit took the scalar body with its
+// range test per point.  kBodyFull drops the masks and, where the cull proved
+// the batch inside the view, the inside test.  The raster is bound by
+// instruction issue (79 % active; 49.6 warp instructions per 32 points, color),
+// so each instruction out of the body shows: with the lane merges, frames took
+// 1B points color 1576 -> 1329 us, 100M flight 897 -> 773, HQS 300M 1135 -> 1066,
+// octree of 2M 46.2 -> 40.9, 15M points in 24 files 84.9 -> 81.5.
+enum Body : int {
+    kBodyScalar = 0,  // one at a time, any w
+    kBodyPair = 1,    // w-safe batches: two per packed instruction
+    kBodyFull = 2     // w-safe whole aligned batches inside the view: no masks, no inside test
+};
+
+// Keeps the smaller key of candidates a and b in a, and drops b, if both are in
+// view on one pixel.
+//
+// A lane's 4 consecutive points of a Morton-ordered batch mostly share a pixel,
+// and each used to probe the CTA's z-cache and issue its own atomic: the L1 data
+// pipe ran at 74 % and held the kernel.  Three merges leave one candidate per
+// lane (wavefronts 74 % -> 36 %, L2 reductions 17.7 M -> 5.9 M per 95 M points),
+// after which instruction issue is the bound.  1B points, color 1576 -> 1500 us;
+// all five merges of 4 points measured 1825, and a warp-wide minimum for
+// candidates on one pixel 1690.  The color payload branches (its 64-bit key
+// costs four instructions that many merges skip: 800M points 1085 against 1111
+// us branchless), the others select (100M flight, index, 843 against 881).
+template <int MODE, int PAYLOAD>
+__device__ __forceinline__ void merge_pair(int a, int b, bool ok[4], const uint32_t pix[4],
+                                           uint32_t wb[4], uint32_t pl[4]) {
+    if (MODE == kModeRaster && PAYLOAD == CR_PAYLOAD_COLOR) {
+        if (ok[a] && ok[b] && pix[a] == pix[b]) {
+            const unsigned long long ka = ((unsigned long long)wb[a] << 32) | pl[a];
+            const unsigned long long kb = ((unsigned long long)wb[b] << 32) | pl[b];
+            if (kb < ka) {
+                wb[a] = wb[b];
+                pl[a] = pl[b];
+            }
+            ok[b] = false;
+        }
+        return;
+    }
+    const bool m = ok[a] && ok[b] && pix[a] == pix[b];
+    if (MODE == kModeHqsDepth) {
+        wb[a] = m ? min(wb[a], wb[b]) : wb[a];
+    } else {
+        // of equal depths the smaller index wins, and a < b holds the smaller
+        const bool less = m && wb[b] < wb[a];
+        wb[a] = less ? wb[b] : wb[a];
+        pl[a] = less ? pl[b] : pl[a];
+    }
+    ok[b] = ok[b] && !m;
+}
+
 // LC: 2 = 10 bit (levels 2-4), 1 = 20 bit (level 1), 0 = 30 bit (level 0).
-// Vectors [vb, ve) of the points [first, first + count) are read as 128-bit vectors starting at the
-// aligned word below `first`; lanes mask the words outside the range.  The
-// next vector is loaded before the current one is processed.  PAIRS (full
-// 10-bit batches that the cull flagged w-safe): points are decoded and
-// projected two at a time with the unchecked reciprocal (project_pair10).
-template <int MODE, int PAYLOAD, int BLOCK, int LC, bool FULL = false, bool PAIRS = false,
-          bool LIT = false>
+// Vectors [vb, ve) of the points [first, first + count) are read as 128-bit
+// vectors starting at the aligned word below `first`; lanes mask the words
+// outside the range.  The next vector is loaded before the current one is
+// processed.
+template <int MODE, int PAYLOAD, int BLOCK, int LC, int BODY, bool LIT>
 __device__ __forceinline__ void run_points(const BatchedLaunch& bl, unsigned long long* zc,
                                            const BatchCtx& c, const PairParams& pp, int64_t first,
                                            int32_t count, bool l0_x12, int vb, int ve) {
-    static_assert(!PAIRS || (FULL && LC == 2), "pairs decode full 10-bit batches");
+    constexpr bool FULL = BODY == kBodyFull;
+    constexpr bool PAIRS = BODY != kBodyScalar;
+    static_assert(!FULL || LC == 2, "whole batches decode at 10 bit");
     PairCol3 pf{};
     if constexpr (PAIRS) pf = PairCol3{f2_pack(c.T12, c.T12), f2_pack(c.T13, c.T13), f2_pack(c.T15, c.T15)};
     constexpr bool kNeedColor = (MODE == kModeHqsColor) || (MODE == kModeRaster && PAYLOAD == CR_PAYLOAD_COLOR);
@@ -297,6 +353,7 @@ __device__ __forceinline__ void run_points(const BatchedLaunch& bl, unsigned lon
     const int nv = min(ve, uvec4 ? min((head + count + 3) >> 2, kPointsPerBatch / 4)
                                  : (head + count + 3) >> 2);
     const uint32_t index0 = (uint32_t)(first - head);  // global index of word 0 of vector v0
+    const uint32_t bias = pixel_bias(c.W);
     const uint4* lo4 = reinterpret_cast<const uint4*>(bl.lo) + v0;
     const uint4* md4 = reinterpret_cast<const uint4*>(bl.md) + v0;
     const uint4* hi4 = reinterpret_cast<const uint4*>(bl.hi) + v0;
@@ -304,13 +361,14 @@ __device__ __forceinline__ void run_points(const BatchedLaunch& bl, unsigned lon
     const uint4 zero = make_uint4(0, 0, 0, 0);
     uint4 n4 = zero, n8 = zero, n12 = zero, ncol = zero;
     PairBatch pb{};
-    if constexpr (PAIRS) pb = pair_batch(c);
+    if constexpr (PAIRS) pb = pair_batch<LC>(c);
     if (vb + (int)threadIdx.x < nv) {
         n4 = ld_stream(lo4 + vb + threadIdx.x);
         if (LC <= 1) n8 = ld_stream(md4 + vb + threadIdx.x);
         if (LC == 0) n12 = ld_stream(hi4 + vb + threadIdx.x);
         if (kNeedColor) ncol = ld_stream(co4 + vb + threadIdx.x);
     }
+#pragma unroll 1
     for (int base = vb; base < nv; base += BLOCK) {
         const int v = base + (int)threadIdx.x;
         const uint4 w4 = n4, w8 = n8, w12 = n12, col = ncol;
@@ -321,30 +379,50 @@ __device__ __forceinline__ void run_points(const BatchedLaunch& bl, unsigned lon
             if (LC == 0) n12 = ld_stream(hi4 + vn);
             if (kNeedColor) ncol = ld_stream(co4 + vn);
         }
-        const int32_t rel0 = 4 * v - head;  // batch-local index of word 0
-        // the reference's thread 0 returns before any point when head != 0
-        const bool lane_live = !uvec4 || (v & 127) != 0;
+        bool ok[4];
+        uint32_t pix[4], wb[4];
+        if constexpr (PAIRS && LC == 2) {
+            project_pair10<LIT, FULL>(pp, pf, pb, c.W, w4.x, w4.y, ok, pix, wb);
+            project_pair10<LIT, FULL>(pp, pf, pb, c.W, w4.z, w4.w, ok + 2, pix + 2, wb + 2);
+        } else if constexpr (PAIRS) {
+#pragma unroll
+            for (int h = 0; h < 4; h += 2) {
+                uint32_t q[2][3];
+                decode_fields<LC>(w4, w8, w12, h, l0_x12, q[0]);
+                decode_fields<LC>(w4, w8, w12, h + 1, l0_x12, q[1]);
+                project_pair<LIT>(pp, pf, pb, c.W,
+                                  f2_pack(__uint2float_rn(q[0][0]), __uint2float_rn(q[1][0])),
+                                  f2_pack(__uint2float_rn(q[0][1]), __uint2float_rn(q[1][1])),
+                                  f2_pack(__uint2float_rn(q[0][2]), __uint2float_rn(q[1][2])),
+                                  ok + h, pix + h, wb + h);
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                uint32_t q[3];
+                decode_fields<LC>(w4, w8, w12, j, l0_x12, q);
+                const float x = decode_axis<LIT>(__uint2float_rn(q[0]), c.sx, c.mnx);
+                const float y = decode_axis<LIT>(__uint2float_rn(q[1]), c.sy, c.mny);
+                const float z = decode_axis<LIT>(__uint2float_rn(q[2]), c.sz, c.mnz);
+                int32_t p;
+                ok[j] = project<false, LIT>(c, x, y, z, p, wb[j]);
+                pix[j] = (uint32_t)p + bias;
+            }
+        }
+        if constexpr (!FULL) {
+            const int32_t rel0 = 4 * v - head;  // batch-local index of word 0
+            // the reference's thread 0 returns before any point when head != 0
+            const bool lane_live = !uvec4 || (v & 127) != 0;
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                ok[j] = ok[j] && (uint32_t)(rel0 + j) < (uint32_t)count && lane_live;
+        }
         if constexpr (MODE == kModeHqsColor) {
             // The lane's 4 consecutive points, in runs of in-view points on one
             // pixel (Morton order puts most of them on the same pixel): project
             // all 4, read the depth of every run start at once (the reads
             // overlap; the depth buffer is read-only in this pass), then sum
             // each run's visible colors and flush it once.
-            int32_t pix[4];
-            uint32_t wb[4];
-            bool ok[4];
-            if constexpr (PAIRS) {
-                project_pair10<LIT>(pp, pf, pb, c.W, w4.x, w4.y, ok, pix, wb);
-                project_pair10<LIT>(pp, pf, pb, c.W, w4.z, w4.w, ok + 2, pix + 2, wb + 2);
-            } else {
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const bool valid = FULL || ((uint32_t)(rel0 + j) < (uint32_t)count && lane_live);
-                    float x, y, z;
-                    decode_point<LC, LIT>(w4, w8, w12, j, c, l0_x12, x, y, z);
-                    ok[j] = project<false, LIT>(c, x, y, z, pix[j], wb[j]) && valid;
-                }
-            }
             bool cont[4];
             float lim[4];
 #pragma unroll
@@ -352,7 +430,7 @@ __device__ __forceinline__ void run_points(const BatchedLaunch& bl, unsigned lon
                 const int jp = j > 0 ? j - 1 : 0;
                 cont[j] = j > 0 && ok[jp] && ok[j] && pix[j] == pix[jp];
                 // color.cs:399-403: visible if depth <= bufferDepth * 1.01
-                lim[j] = ok[j] && !cont[j] ? fmul(__uint_as_float(__ldg(bl.depth + pix[j])), 1.01f) : 0.0f;
+                lim[j] = ok[j] && !cont[j] ? fmul(__uint_as_float(__ldg(bl.depth + (pix[j] - bias))), 1.01f) : 0.0f;
             }
             uint32_t rg = 0u, bc = 0u;
             float run_lim = 0.0f;
@@ -361,7 +439,7 @@ __device__ __forceinline__ void run_points(const BatchedLaunch& bl, unsigned lon
                 const int jp = j > 0 ? j - 1 : 0;
                 // a run that ends inside the vector goes straight to the
                 // accumulators; only the lane's last run joins the warp merge
-                if (j > 0 && ok[jp] && !cont[j] && bc != 0u) hqs_color_add(bl, pix[jp], rg, bc);
+                if (j > 0 && ok[jp] && !cont[j] && bc != 0u) hqs_color_add(bl, pix[jp] - bias, rg, bc);
                 if (!cont[j]) {
                     rg = bc = 0u;
                     run_lim = lim[j];
@@ -373,47 +451,28 @@ __device__ __forceinline__ void run_points(const BatchedLaunch& bl, unsigned lon
                     bc += __byte_perm(color, 0x00010000u, 0x7642);
                 }
             }
-            hqs_color_flush(bl, ok[3] && bc != 0u, pix[3], rg, bc);
-        } else if constexpr (PAIRS) {
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                int32_t pix[2];
-                uint32_t wb[2];
-                bool ok[2];
-                project_pair10<LIT>(pp, pf, pb, c.W, h ? w4.z : w4.x, h ? w4.w : w4.y, ok, pix, wb);
-#pragma unroll
-                for (int k = 0; k < 2; k++) {
-                    const int j = 2 * h + k;
-                    const uint32_t idx = index0 + 4u * (uint32_t)v + (uint32_t)j;
-                    const uint32_t color = kNeedColor ? u4get(col, j) : 0u;
-                    const uint32_t payload = (PAYLOAD == CR_PAYLOAD_COLOR) ? color : idx;
-                    Emit<MODE>::run(bl, zc, ok[k], pix[k], wb[k], payload, color);
-                }
-            }
+            hqs_color_flush(bl, ok[3] && bc != 0u, pix[3] - bias, rg, bc);
         } else {
+            uint32_t pl[4];
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const bool valid = FULL || ((uint32_t)(rel0 + j) < (uint32_t)count && lane_live);
-                const uint32_t idx = index0 + 4u * (uint32_t)v + (uint32_t)j;
-                float x, y, z;
-                decode_point<LC, LIT>(w4, w8, w12, j, c, l0_x12, x, y, z);
-                int32_t pix;
-                uint32_t wbits;
-                const bool ok = project<false, LIT>(c, x, y, z, pix, wbits) && valid;
-                const uint32_t color = kNeedColor ? u4get(col, j) : 0u;
-                const uint32_t payload = (PAYLOAD == CR_PAYLOAD_COLOR) ? color : (uint32_t)idx;
-                Emit<MODE>::run(bl, zc, ok, pix, wbits, payload, color);
-            }
+            for (int j = 0; j < 4; j++)
+                pl[j] = PAYLOAD == CR_PAYLOAD_COLOR ? u4get(col, j) : index0 + 4u * (uint32_t)v + (uint32_t)j;
+            merge_pair<MODE, PAYLOAD>(0, 1, ok, pix, wb, pl);
+            merge_pair<MODE, PAYLOAD>(2, 3, ok, pix, wb, pl);
+            merge_pair<MODE, PAYLOAD>(0, 2, ok, pix, wb, pl);
+#pragma unroll
+            for (int j = 0; j < 4; j++) Emit<MODE>::run(bl, zc, bias, ok[j], pix[j], wb[j], pl[j]);
         }
     }
 }
 
-// The HQS color pass's 10-bit instance is held to 48 registers, at which 10
-// CTAs of 128 threads stay resident per SM (its uncapped 51 leave 9 CTAs per
-// SM; measured 1 % slower).  UNCAPPED: the many-file literal instance, which
-// spills under the cap.
+// Resident CTAs per SM of the HQS color pass: 9 for the 10-bit list (56
+// registers; HQS 300M 1067 us, against 1077 at 10 CTAs, where the masked pair
+// body spills, and 1069 at 8), 8 for the 20/30-bit list (uncapped it takes 90
+// registers, 5 CTAs).  UNCAPPED: the many-file literal instance, which spills
+// under the cap.
 template <int MODE, int BLOCK, int LIST, bool UNCAPPED = false>
-constexpr int kMinBlocks = MODE == kModeHqsColor && LIST == 0 && !UNCAPPED ? 1280 / BLOCK : 0;
+constexpr int kMinBlocks = MODE != kModeHqsColor || UNCAPPED ? 0 : (LIST == 0 ? 9 : 8) * 128 / BLOCK;
 
 // How a launch hands out `nitems` list items to its CTAs: the first `whole`
 // items as one unit each, every later item as `parts` units of `part_vectors`
@@ -476,7 +535,7 @@ __global__ void __launch_bounds__(BLOCK, (kMinBlocks<MODE, BLOCK, LIST, MANY && 
     const WorkSplit ws = split_work<BLOCK>(nitems, gridDim.x, bl.node_slices);
     if (blockIdx.x < ws.units) {
         if (MODE != kModeHqsColor)
-            for (int i = threadIdx.x; i < kZCacheSlots; i += BLOCK) s_zc[i] = 0xFFFFFFFFull;
+            for (int i = threadIdx.x; i < kZCacheSlots; i += BLOCK) s_zc[i] = kZCacheEmpty;
         // the first unit is the CTA's own number; the cursor hands out the rest
         if (threadIdx.x == 0) s_item[0] = blockIdx.x;
         __syncthreads();
@@ -497,7 +556,7 @@ __global__ void __launch_bounds__(BLOCK, (kMinBlocks<MODE, BLOCK, LIST, MANY && 
             const uint32_t item =
                 bl.scratch[kScratchHead + (LIST == 0 ? (int64_t)wi : bl.list_cap - 1 - (int64_t)wi)];
             const uint32_t b = item & (bl.node_slices ? kItemNodeMask : kItemBatchMask);
-            const int level = (int)(item >> 29);
+            const int level = (int)(item >> 29);  // levels 2-4 + kLevelInside: inside the view
 
             const int4* r4 = reinterpret_cast<const int4*>(bl.batches + b);
             const int4 ra = __ldg(r4), rc = __ldg(r4 + 1), rd = __ldg(r4 + 2);
@@ -529,22 +588,28 @@ __global__ void __launch_bounds__(BLOCK, (kMinBlocks<MODE, BLOCK, LIST, MANY && 
             }
             c.Wf = (float)vp.W; c.Hf = (float)vp.H; c.W = vp.W;
             const bool l0_x12 = (bl.quirks & CR_QUIRK_L0_X12) != 0;
-            // full, vector-aligned batches whose w range is proven safe (nearly
-            // all) skip the per-point range test and decode in pairs; the rest
-            // take the general body
-            // (node slices of kNodeSlice points qualify too: whole vectors for
-            // every thread, as the full path needs)
-            if (LIST == 0 && (item & kItemWSafe) &&
-                (count == kPointsPerBatch ||
-                 (kNodeSlice % (4 * BLOCK) == 0 && bl.node_slices && count == kNodeSlice)) &&
-                (first & 3) == 0 && pair_batch_exact(c))
-                run_points<MODE, PAYLOAD, BLOCK, 2, true, true, LIT>(bl, s_zc, c, pp, first, count, l0_x12, vb, ve);
-            else if (LIST == 0)
-                run_points<MODE, PAYLOAD, BLOCK, 2, false, false, LIT>(bl, s_zc, c, pp, first, count, l0_x12, vb, ve);
-            else if (level == 1)
-                run_points<MODE, PAYLOAD, BLOCK, 1, false, false, LIT>(bl, s_zc, c, pp, first, count, l0_x12, vb, ve);
-            else
-                run_points<MODE, PAYLOAD, BLOCK, 0, false, false, LIT>(bl, s_zc, c, pp, first, count, l0_x12, vb, ve);
+            // whole vector-aligned batches inside the view (node slices of
+            // kNodeSlice points too: whole vectors for every thread) take the
+            // body without masks, other w-safe ones the pair body, the rest the
+            // scalar body (see Body)
+            const bool safe = (item & kItemWSafe) != 0;
+            if (LIST == 0 && safe && pair_batch_exact(c)) {
+                if (level >= 2 + kLevelInside &&
+                    (count == kPointsPerBatch ||
+                     (kNodeSlice % (4 * BLOCK) == 0 && bl.node_slices && count == kNodeSlice)) &&
+                    (first & 3) == 0)
+                    run_points<MODE, PAYLOAD, BLOCK, 2, kBodyFull, LIT>(bl, s_zc, c, pp, first, count, l0_x12, vb, ve);
+                else
+                    run_points<MODE, PAYLOAD, BLOCK, 2, kBodyPair, LIT>(bl, s_zc, c, pp, first, count, l0_x12, vb, ve);
+            } else if (LIST == 0) {
+                run_points<MODE, PAYLOAD, BLOCK, 2, kBodyScalar, LIT>(bl, s_zc, c, pp, first, count, l0_x12, vb, ve);
+            } else if (level == 1) {
+                if (safe) run_points<MODE, PAYLOAD, BLOCK, 1, kBodyPair, LIT>(bl, s_zc, c, pp, first, count, l0_x12, vb, ve);
+                else run_points<MODE, PAYLOAD, BLOCK, 1, kBodyScalar, LIT>(bl, s_zc, c, pp, first, count, l0_x12, vb, ve);
+            } else {
+                if (safe) run_points<MODE, PAYLOAD, BLOCK, 0, kBodyPair, LIT>(bl, s_zc, c, pp, first, count, l0_x12, vb, ve);
+                else run_points<MODE, PAYLOAD, BLOCK, 0, kBodyScalar, LIT>(bl, s_zc, c, pp, first, count, l0_x12, vb, ve);
+            }
             __syncthreads();
             buf ^= 1;
         }
@@ -583,7 +648,7 @@ __global__ void __launch_bounds__(BLOCK) k_plain(PlainParams pp, const uint4* __
     // VARIANT 1: per warp a 4096-bit map of the pixels its in-view lanes hit
     __shared__ uint32_t s_bits[VARIANT == 1 ? BLOCK / 32 * 128 : 1];
     if (VARIANT == 0) {
-        for (int i = threadIdx.x; i < kZCacheSlots; i += BLOCK) s_zc[i] = 0xFFFFFFFFull;
+        for (int i = threadIdx.x; i < kZCacheSlots; i += BLOCK) s_zc[i] = kZCacheEmpty;
         __syncthreads();
     }
     if (VARIANT == 1) {
@@ -602,7 +667,7 @@ __global__ void __launch_bounds__(BLOCK) k_plain(PlainParams pp, const uint4* __
         const bool ok = project<false, LIT>(c, __uint_as_float(p.x), __uint_as_float(p.y),
                                             __uint_as_float(p.z), pix, wbits) && act;
         if (VARIANT == 0) {
-            Emit<kModeRaster>::run(bl, s_zc, ok, pix, wbits, p.w, 0u);
+            Emit<kModeRaster>::run(bl, s_zc, 0u, ok, (uint32_t)pix, wbits, p.w);
             continue;
         }
         // wbits = floatBitsToInt(pos.w), positive for every point in view

@@ -287,7 +287,7 @@ __device__ __forceinline__ void mv_raster_items(const MVArgs& a) {
         *reinterpret_cast<volatile uint32_t*>(a.scratch + (LIST == 0 ? kItemCount : kItemCount2));
     if (nitems == 0) return;
     const uint4* items = reinterpret_cast<const uint4*>(a.scratch + kScratchHead);
-    for (int i = threadIdx.x; i < kZCacheSlots; i += BLOCK) s_zc[i] = 0xFFFFFFFFull;
+    for (int i = threadIdx.x; i < kZCacheSlots; i += BLOCK) s_zc[i] = kZCacheEmpty;
     if (threadIdx.x == 0) s_item[0] = atomicAdd(cursor, 1u);
     __syncthreads();
     const bool l0_x12 = (a.quirks & CR_QUIRK_L0_X12) != 0;
