@@ -231,6 +231,57 @@ __device__ __forceinline__ int64_t points_in_batch(int32_t num_points, int32_t f
     return n < 0 ? 0 : n;
 }
 
+// How a launch hands out `nitems` list items to its CTAs: the first `whole`
+// items as one unit each, every later item as `parts` units of `part_vectors`
+// vectors.
+//
+// A CTA walks a whole batch in 20 serial steps of 512 points, about 16 us alone
+// and 30 us on a full SM, so a frame with few items left most SMs idle and
+// every frame ended in a wave of whole batches.  The last item per CTA goes out
+// in fifths (4 steps), and in tenths or single steps while there would be fewer
+// than two parts per CTA.  Items before those stay whole: a unit costs about a
+// step (cursor, record and first vectors, one after the other), and cutting
+// every batch measured 3-9 % slower on the 100M-point flight.  Frames, whole
+// batches -> parts: 50k points 32.9 -> 22.6 us, octree of 2M 54.2 -> 46.2,
+// 15M points in 24 files 121 -> 85, 100M-point flight (5 poses) 930 -> 897; a
+// billion points 1572 -> 1576 (its last wave is small beside its length).
+struct WorkSplit {
+    uint32_t whole, parts, units;
+    int part_vectors;
+};
+constexpr int kAllVectors = 1 << 30;
+
+template <int BLOCK>
+__device__ __forceinline__ WorkSplit split_work(uint32_t nitems, uint32_t ctas, bool node_slices) {
+    // parts are whole steps of the CTA: 2,560 vectors of a batch (640 of a
+    // node slice) are `steps` steps of BLOCK vectors
+    const uint32_t steps = (node_slices ? kNodeSlice : kPointsPerBatch) / (4 * BLOCK);
+    uint32_t parts = steps % 5 == 0 ? 5 : 1;
+    if (nitems * parts < 2 * ctas) parts = steps % 10 == 0 ? 10 : steps;
+    if (nitems * parts < 2 * ctas) parts = steps;
+    WorkSplit w;
+    w.parts = parts > 0 ? parts : 1;
+    w.part_vectors = (int)(max(steps / w.parts, 1u) * BLOCK);
+    const uint32_t split = min(nitems, ctas);
+    w.whole = nitems - split;
+    w.units = w.whole + split * w.parts;
+    return w;
+}
+
+// The list item of a unit and its range of vectors.
+__device__ __forceinline__ void unit_range(const WorkSplit& ws, uint32_t unit, uint32_t* item, int* vb,
+                                           int* ve) {
+    *item = unit;
+    *vb = 0;
+    *ve = kAllVectors;
+    if (unit < ws.whole) return;
+    const uint32_t k = (unit - ws.whole) / ws.parts, part = (unit - ws.whole) - k * ws.parts;
+    *item = ws.whole + k;
+    *vb = (int)part * ws.part_vectors;
+    // the last part of an unaligned batch takes its extra vector too
+    if (part + 1 != ws.parts) *ve = *vb + ws.part_vectors;
+}
+
 struct BatchCtx {
     float mnx, mny, mnz;
     float sx, sy, sz;
@@ -288,6 +339,43 @@ __device__ __forceinline__ bool zcache_rejects(const unsigned long long* zc, uin
                                                uint32_t tag, uint32_t wbits) {
     const unsigned long long e = zc[slot];
     return (uint32_t)e == tag && wbits > (uint32_t)(e >> 32);
+}
+
+// Keeps the smaller key of candidates a and b in a, and drops b, if both are in
+// view on one pixel.
+//
+// A lane's 4 consecutive points of a Morton-ordered batch mostly share a pixel,
+// and each used to probe the CTA's z-cache and issue its own atomic: the L1 data
+// pipe ran at 74 % and held the kernel.  Three merges leave one candidate per
+// lane (wavefronts 74 % -> 36 %, L2 reductions 17.7 M -> 5.9 M per 95 M points),
+// after which instruction issue is the bound.  1B points, color 1576 -> 1500 us;
+// all five merges of 4 points measured 1825, and a warp-wide minimum for
+// candidates on one pixel 1690.  The color payload branches (its 64-bit key
+// costs four instructions that many merges skip: 800M points 1085 against 1111
+// us branchless), the others select (100M flight, index, 843 against 881).
+// TIES: payloads are colors, so equal depths compare them; indices rise with the
+// point, and of equal depths a holds the smaller one (merges take a < b).  The
+// HQS depth pass has no payload and drops the select.
+template <bool TIES>
+__device__ __forceinline__ void merge_pair(int a, int b, bool ok[4], const uint32_t pix[4],
+                                           uint32_t wb[4], uint32_t pl[4]) {
+    if (TIES) {
+        if (ok[a] && ok[b] && pix[a] == pix[b]) {
+            const unsigned long long ka = ((unsigned long long)wb[a] << 32) | pl[a];
+            const unsigned long long kb = ((unsigned long long)wb[b] << 32) | pl[b];
+            if (kb < ka) {
+                wb[a] = wb[b];
+                pl[a] = pl[b];
+            }
+            ok[b] = false;
+        }
+        return;
+    }
+    const bool m = ok[a] && ok[b] && pix[a] == pix[b];
+    const bool less = m && wb[b] < wb[a];
+    wb[a] = less ? wb[b] : wb[a];
+    pl[a] = less ? pl[b] : pl[a];
+    ok[b] = ok[b] && !m;
 }
 
 // Clip-space position of a decoded point (render.cs:399-401).  LIT

@@ -286,45 +286,6 @@ enum Body : int {
     kBodyFull = 2     // w-safe whole aligned batches inside the view: no masks, no inside test
 };
 
-// Keeps the smaller key of candidates a and b in a, and drops b, if both are in
-// view on one pixel.
-//
-// A lane's 4 consecutive points of a Morton-ordered batch mostly share a pixel,
-// and each used to probe the CTA's z-cache and issue its own atomic: the L1 data
-// pipe ran at 74 % and held the kernel.  Three merges leave one candidate per
-// lane (wavefronts 74 % -> 36 %, L2 reductions 17.7 M -> 5.9 M per 95 M points),
-// after which instruction issue is the bound.  1B points, color 1576 -> 1500 us;
-// all five merges of 4 points measured 1825, and a warp-wide minimum for
-// candidates on one pixel 1690.  The color payload branches (its 64-bit key
-// costs four instructions that many merges skip: 800M points 1085 against 1111
-// us branchless), the others select (100M flight, index, 843 against 881).
-template <int MODE, int PAYLOAD>
-__device__ __forceinline__ void merge_pair(int a, int b, bool ok[4], const uint32_t pix[4],
-                                           uint32_t wb[4], uint32_t pl[4]) {
-    if (MODE == kModeRaster && PAYLOAD == CR_PAYLOAD_COLOR) {
-        if (ok[a] && ok[b] && pix[a] == pix[b]) {
-            const unsigned long long ka = ((unsigned long long)wb[a] << 32) | pl[a];
-            const unsigned long long kb = ((unsigned long long)wb[b] << 32) | pl[b];
-            if (kb < ka) {
-                wb[a] = wb[b];
-                pl[a] = pl[b];
-            }
-            ok[b] = false;
-        }
-        return;
-    }
-    const bool m = ok[a] && ok[b] && pix[a] == pix[b];
-    if (MODE == kModeHqsDepth) {
-        wb[a] = m ? min(wb[a], wb[b]) : wb[a];
-    } else {
-        // of equal depths the smaller index wins, and a < b holds the smaller
-        const bool less = m && wb[b] < wb[a];
-        wb[a] = less ? wb[b] : wb[a];
-        pl[a] = less ? pl[b] : pl[a];
-    }
-    ok[b] = ok[b] && !m;
-}
-
 // LC: 2 = 10 bit (levels 2-4), 1 = 20 bit (level 1), 0 = 30 bit (level 0).
 // Vectors [vb, ve) of the points [first, first + count) are read as 128-bit
 // vectors starting at the aligned word below `first`; lanes mask the words
@@ -457,9 +418,10 @@ __device__ __forceinline__ void run_points(const BatchedLaunch& bl, unsigned lon
 #pragma unroll
             for (int j = 0; j < 4; j++)
                 pl[j] = PAYLOAD == CR_PAYLOAD_COLOR ? u4get(col, j) : index0 + 4u * (uint32_t)v + (uint32_t)j;
-            merge_pair<MODE, PAYLOAD>(0, 1, ok, pix, wb, pl);
-            merge_pair<MODE, PAYLOAD>(2, 3, ok, pix, wb, pl);
-            merge_pair<MODE, PAYLOAD>(0, 2, ok, pix, wb, pl);
+            constexpr bool kTies = MODE == kModeRaster && PAYLOAD == CR_PAYLOAD_COLOR;
+            merge_pair<kTies>(0, 1, ok, pix, wb, pl);
+            merge_pair<kTies>(2, 3, ok, pix, wb, pl);
+            merge_pair<kTies>(0, 2, ok, pix, wb, pl);
 #pragma unroll
             for (int j = 0; j < 4; j++) Emit<MODE>::run(bl, zc, bias, ok[j], pix[j], wb[j], pl[j]);
         }
@@ -473,43 +435,6 @@ __device__ __forceinline__ void run_points(const BatchedLaunch& bl, unsigned lon
 // under the cap.
 template <int MODE, int BLOCK, int LIST, bool UNCAPPED = false>
 constexpr int kMinBlocks = MODE != kModeHqsColor || UNCAPPED ? 0 : (LIST == 0 ? 9 : 8) * 128 / BLOCK;
-
-// How a launch hands out `nitems` list items to its CTAs: the first `whole`
-// items as one unit each, every later item as `parts` units of `part_vectors`
-// vectors.
-//
-// A CTA walks a whole batch in 20 serial steps of 512 points, about 16 us alone
-// and 30 us on a full SM, so a frame with few items left most SMs idle and
-// every frame ended in a wave of whole batches.  The last item per CTA goes out
-// in fifths (4 steps), and in tenths or single steps while there would be fewer
-// than two parts per CTA.  Items before those stay whole: a unit costs about a
-// step (cursor, record and first vectors, one after the other), and cutting
-// every batch measured 3-9 % slower on the 100M-point flight.  Frames, whole
-// batches -> parts: 50k points 32.9 -> 22.6 us, octree of 2M 54.2 -> 46.2,
-// 15M points in 24 files 121 -> 85, 100M-point flight (5 poses) 930 -> 897; a
-// billion points 1572 -> 1576 (its last wave is small beside its length).
-struct WorkSplit {
-    uint32_t whole, parts, units;
-    int part_vectors;
-};
-constexpr int kAllVectors = 1 << 30;
-
-template <int BLOCK>
-__device__ __forceinline__ WorkSplit split_work(uint32_t nitems, uint32_t ctas, int node_slices) {
-    // parts are whole steps of the CTA: 2,560 vectors of a batch (640 of a
-    // node slice) are `steps` steps of BLOCK vectors
-    const uint32_t steps = (node_slices ? kNodeSlice : kPointsPerBatch) / (4 * BLOCK);
-    uint32_t parts = steps % 5 == 0 ? 5 : 1;
-    if (nitems * parts < 2 * ctas) parts = steps % 10 == 0 ? 10 : steps;
-    if (nitems * parts < 2 * ctas) parts = steps;
-    WorkSplit w;
-    w.parts = parts > 0 ? parts : 1;
-    w.part_vectors = (int)(max(steps / w.parts, 1u) * BLOCK);
-    const uint32_t split = min(nitems, ctas);
-    w.whole = nitems - split;
-    w.units = w.whole + split * w.parts;
-    return w;
-}
 
 // LIST 0: the 10-bit items (front of the list region), LIST 1: the 20/30-bit
 // items (back of the region).  Each list runs in its own instance, so the
@@ -532,7 +457,7 @@ __global__ void __launch_bounds__(BLOCK, (kMinBlocks<MODE, BLOCK, LIST, MANY && 
                                                : (MODE == kModeHqsColor ? kCursor3 : kCursor2));
     const uint32_t nitems =
         *reinterpret_cast<volatile uint32_t*>(bl.scratch + (LIST == 0 ? kItemCount : kItemCount2));
-    const WorkSplit ws = split_work<BLOCK>(nitems, gridDim.x, bl.node_slices);
+    const WorkSplit ws = split_work<BLOCK>(nitems, gridDim.x, bl.node_slices != 0);
     if (blockIdx.x < ws.units) {
         if (MODE != kModeHqsColor)
             for (int i = threadIdx.x; i < kZCacheSlots; i += BLOCK) s_zc[i] = kZCacheEmpty;
@@ -544,15 +469,9 @@ __global__ void __launch_bounds__(BLOCK, (kMinBlocks<MODE, BLOCK, LIST, MANY && 
             const uint32_t unit = s_item[buf];
             if (unit >= ws.units) break;
             if (threadIdx.x == 0) s_item[buf ^ 1] = gridDim.x + atomicAdd(cursor, 1u);
-            uint32_t wi = unit, part = 0;
-            int vb = 0, ve = kAllVectors;
-            if (unit >= ws.whole) {
-                wi = ws.whole + (unit - ws.whole) / ws.parts;
-                part = (unit - ws.whole) % ws.parts;
-                vb = (int)part * ws.part_vectors;
-                // the last part of an unaligned batch takes its extra vector too
-                ve = part + 1 == ws.parts ? kAllVectors : vb + ws.part_vectors;
-            }
+            uint32_t wi;
+            int vb, ve;
+            unit_range(ws, unit, &wi, &vb, &ve);
             const uint32_t item =
                 bl.scratch[kScratchHead + (LIST == 0 ? (int64_t)wi : bl.list_cap - 1 - (int64_t)wi)];
             const uint32_t b = item & (bl.node_slices ? kItemNodeMask : kItemBatchMask);

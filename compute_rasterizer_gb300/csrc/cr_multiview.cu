@@ -4,13 +4,14 @@
 //
 //   k_mv_cull    one thread per (batch, view group): frustum test and
 //                precision level per view; appends {batch, group, visible
-//                mask, 3-bit level per view, w-safe bit per view at 24 + s}
-//                to a work list.
-//   k_mv_raster  persistent CTAs pull (batch, group) items, read the batch's
-//                points once with 128-bit loads, decode them, and project and
-//                splat every point into each visible view of the group at that
-//                view's own level, through the per-CTA z-cache (tags are the
-//                view's word offset plus the pixel id).
+//                mask, 3-bit level per view (5-7: levels 2-4 inside the view),
+//                w-safe bit per view at 24 + s} to a work list.
+//   k_mv_raster  persistent CTAs pull (batch, group) items (the last ones in
+//                parts), read the batch's points once with 128-bit loads,
+//                decode them in pairs, and project and splat every point into
+//                each visible view of the group at that view's own level,
+//                through the per-CTA z-cache (tags are the view's word offset
+//                plus the pixel id).
 //   k_mv_resolve every view's pixels (grid y = view), fused re-clear.
 // The arithmetic is the single-view kernels' (cr_device.cuh), so each view's
 // framebuffer equals a cr_render of that view alone, bit for bit.
@@ -45,7 +46,12 @@ struct MVArgs {
     const uint32_t* pairs;  // per group: bit s = views s, s + 1 share rows y and w (or NULL)
 };
 
-constexpr int kSlotWords = 16;  // per view slot in shared memory: T[12], Wf, Hf, W, fb_off
+// Per view slot in shared memory: rows w, x and y of T (4 uniforms each, in the
+// order of the products), Wf, Hf, W, the word offset less pixel_bias(W) (see
+// there): four 128-bit reads per view and 4 points.  The packed operations want
+// each uniform twice; slots that hold them so (eight reads) were slower, the L1
+// data pipe being the second bound (200M points, 64 views 7190 us against 6810).
+enum : int { kRowW = 0, kRowX = 4, kRowY = 8, kSize = 12, kInts = 14, kSlotWords = 16 };
 
 // The 12 transform entries of a view's T that the projection uses.
 __host__ __device__ inline void mv_file_from_rec(const FileRec& r, MVFile* o) {
@@ -112,14 +118,15 @@ __global__ void __launch_bounds__(256) k_mv_cull(const MVView* __restrict__ view
                 const int level = precision_level(vw.P, f.VW, vw.W, vw.H, mnx, mny, mnz, mxx, mxy, mxz);
                 if (lod_skip_level > 0 && level >= lod_skip_level) continue;  // nodes/render.cs:273
                 vismask |= 1u << s;
-                levels |= (uint32_t)level << (3 * s);
-                // bit 24 + s: view s's clip w is proven to lie in [2^-120, 2^120]
-                float tw[16];
-                tw[3] = f.T[2];
-                tw[7] = f.T[5];
-                tw[11] = f.T[8];
-                tw[15] = f.T[11];
-                if (w_safe(tw, mnx, mny, mnz, mxx, mxy, mxz)) levels |= 1u << (24 + s);
+                // bit 24 + s: view s's clip w is proven to lie in [2^-120, 2^120];
+                // levels 2-4 + kLevelInside: every point projects inside view s
+                float t[16];
+#pragma unroll
+                for (int k = 0; k < 12; k++) t[k < 3 ? (k == 2 ? 3 : k) : (k / 3) * 4 + (k % 3 == 2 ? 3 : k % 3)] = f.T[k];
+                const bool safe = w_safe(t, mnx, mny, mnz, mxx, mxy, mxz);
+                const bool inside = safe && level >= 2 && all_inside(t, mnx, mny, mnz, mxx, mxy, mxz);
+                levels |= (uint32_t)(inside ? level + kLevelInside : level) << (3 * s);
+                if (safe) levels |= 1u << (24 + s);
             }
             keep = vismask != 0;
             item = make_uint4((uint32_t)b, (uint32_t)g, vismask, levels);
@@ -154,124 +161,206 @@ __global__ void __launch_bounds__(256) k_mv_cull(const MVView* __restrict__ view
     }
 }
 
+// tag: the framebuffer word of the candidate's pixel.  Atomic and cache entry
+// are predicated, not branched around: three candidates in four warps have one.
 __device__ __forceinline__ void emit_mv(unsigned long long* fbs, unsigned long long* zc, bool ok,
-                                        int32_t pix, uint32_t fb_off, uint32_t wbits,
-                                        uint32_t payload) {
-    const uint32_t tag = fb_off + (uint32_t)pix;
+                                        uint32_t tag, uint32_t wbits, uint32_t payload) {
     const uint32_t slot = zslot(tag);
     const bool cand = ok && !zcache_rejects(zc, slot, tag, wbits);
-    if (__any_sync(kFull, cand) && cand)
-        submit_min<unsigned long long>(fbs + tag, zc, slot, tag,
-                                       ((unsigned long long)wbits << 32) | payload, wbits);
+    const unsigned long long key = ((unsigned long long)wbits << 32) | payload;
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.u32 p, %0, 0;\n"
+        " @p red.relaxed.gpu.global.min.u64 [%1], %2;\n @p st.shared.v2.u32 [%3], {%4, %5};\n}"
+        :: "r"((uint32_t)cand), "l"(fbs + tag), "l"(key),
+           "r"((uint32_t)__cvta_generic_to_shared(zc + slot)), "r"(tag), "r"(wbits)
+        : "memory");
 }
 
+// The thread's 4 decoded points as two pairs (points 0, 1 and 2, 3).
 struct Decoded {
-    float x[4], y[4], z[4];
+    uint64_t x[2], y[2], z[2];
 };
 
 // Decodes the thread's 4 points at level class LC (2: 10 bit, 1: 20 bit, 0: 30 bit).
 __device__ __forceinline__ void decode4(int LC, const uint4& w4, const uint4& w8, const uint4& w12,
                                         float mnx, float mny, float mnz, const float* s,
                                         bool l0_x12, Decoded& o) {
+    const uint64_t MX = f2_pack(mnx, mnx), MY = f2_pack(mny, mny), MZ = f2_pack(mnz, mnz);
+    const int k = LC == 2 ? 0 : 3;
+    const uint64_t SX = f2_pack(s[k], s[k]), SY = f2_pack(s[k + 1], s[k + 1]), SZ = f2_pack(s[k + 2], s[k + 2]);
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-        const uint32_t a = u4get(w4, j);
-        if (LC == 2) {
-            o.x[j] = __fmaf_rn(small_u2f(a & 1023u), s[0], mnx);
-            o.y[j] = __fmaf_rn(small_u2f((a >> 10) & 1023u), s[1], mny);
-            o.z[j] = __fmaf_rn(small_u2f((a >> 20) & 1023u), s[2], mnz);
-        } else {
-            const uint32_t b = u4get(w8, j);
-            uint32_t X = ((a & 1023u) << 20) | ((b & 1023u) << 10);
-            uint32_t Y = (((a >> 10) & 1023u) << 20) | (((b >> 10) & 1023u) << 10);
-            uint32_t Z = (((a >> 20) & 1023u) << 20) | (((b >> 20) & 1023u) << 10);
-            if (LC == 0) {
-                const uint32_t h = u4get(w12, j);
-                uint32_t x12 = h & 1023u, y12 = (h >> 10) & 1023u, z12 = (h >> 20) & 1023u;
-                if (l0_x12) { y12 = x12; z12 = x12; }
-                X |= x12; Y |= y12; Z |= z12;
+    for (int h = 0; h < 2; h++) {
+        uint32_t q[2][3];
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const uint32_t a = u4get(w4, 2 * h + j);
+            if (LC == 2) {
+                q[j][0] = a & 1023u;
+                q[j][1] = (a >> 10) & 1023u;
+                q[j][2] = (a >> 20) & 1023u;
+                continue;
             }
-            o.x[j] = __fmaf_rn(__uint2float_rn(X), s[3], mnx);
-            o.y[j] = __fmaf_rn(__uint2float_rn(Y), s[4], mny);
-            o.z[j] = __fmaf_rn(__uint2float_rn(Z), s[5], mnz);
+            const uint32_t b = u4get(w8, 2 * h + j);
+            q[j][0] = ((a & 1023u) << 20) | ((b & 1023u) << 10);
+            q[j][1] = (((a >> 10) & 1023u) << 20) | (((b >> 10) & 1023u) << 10);
+            q[j][2] = (((a >> 20) & 1023u) << 20) | (((b >> 20) & 1023u) << 10);
+            if (LC == 0) {
+                const uint32_t c = u4get(w12, 2 * h + j);
+                uint32_t x12 = c & 1023u, y12 = (c >> 10) & 1023u, z12 = (c >> 20) & 1023u;
+                if (l0_x12) { y12 = x12; z12 = x12; }
+                q[j][0] |= x12; q[j][1] |= y12; q[j][2] |= z12;
+            }
         }
+        o.x[h] = f2_fma(f2_pack(__uint2float_rn(q[0][0]), __uint2float_rn(q[1][0])), SX, MX);
+        o.y[h] = f2_fma(f2_pack(__uint2float_rn(q[0][1]), __uint2float_rn(q[1][1])), SY, MY);
+        o.z[h] = f2_fma(f2_pack(__uint2float_rn(q[0][2]), __uint2float_rn(q[1][2])), SZ, MZ);
     }
 }
 
 __device__ __forceinline__ int level_class(int level) { return level >= 2 ? 2 : level; }
 
-// Projects the 4 decoded points into the view in shared-memory slot `sv` and
-// splats them.  The slot holds T[12], then (Wf, Hf, W, fb_off), 16-byte aligned.
-template <int PAYLOAD, bool SAFE>
-__device__ __forceinline__ void splat_view(const MVArgs& a, unsigned long long* zc, const float* sv,
-                                           const Decoded& d, uint32_t valid_mask, uint32_t idx0,
-                                           const uint4& col) {
-    const float4 t0 = reinterpret_cast<const float4*>(sv)[0];
-    const float4 t1 = reinterpret_cast<const float4*>(sv)[1];
-    const float4 t2 = reinterpret_cast<const float4*>(sv)[2];
-    const float4 t3 = reinterpret_cast<const float4*>(sv)[3];
-    BatchCtx c;
-    c.T0 = t0.x; c.T1 = t0.y; c.T3 = t0.z; c.T4 = t0.w;
-    c.T5 = t1.x; c.T7 = t1.y; c.T8 = t1.z; c.T9 = t1.w;
-    c.T11 = t2.x; c.T12 = t2.y; c.T13 = t2.z; c.T15 = t2.w;
-    c.Wf = t3.x;
-    c.Hf = t3.y;
-    c.W = __float_as_int(t3.z);
-    const uint32_t fb_off = __float_as_uint(t3.w);
+// Row `row` of the slot's transform for the thread's 4 points.
+__device__ __forceinline__ void project_row(const float* sv, int row, const Decoded& d, uint64_t o[2]) {
+    const float4 t = *reinterpret_cast<const float4*>(sv + row);
+    const uint64_t tx = f2_pack(t.x, t.x), ty = f2_pack(t.y, t.y), tz = f2_pack(t.z, t.z), tw = f2_pack(t.w, t.w);
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-        int32_t pix;
-        uint32_t wbits;
-        const bool ok = project<SAFE>(c, d.x[j], d.y[j], d.z[j], pix, wbits) && ((valid_mask >> j) & 1u);
-        const uint32_t payload = (PAYLOAD == CR_PAYLOAD_COLOR) ? u4get(col, j) : idx0 + (uint32_t)j;
-        emit_mv(a.fbs, zc, ok, pix, fb_off, wbits, payload);
+    for (int h = 0; h < 2; h++)
+        o[h] = f2_fma(tz, d.z[h], f2_fma(ty, d.y[h], f2_fma(tx, d.x[h], tw)));
+}
+
+// int(f) as float bits less 0x4B000000 (see pixel_bias), f = (q * 0.5 + 0.5) * size,
+// from NQ = -q; *in: |q| <= 1.
+template <bool INSIDE>
+__device__ __forceinline__ void screen_axis(const uint64_t NQ[2], uint64_t size, bool in[4],
+                                            uint32_t bits[4]) {
+    constexpr uint64_t kHalf = 0x3F0000003F000000ull, kNHalf = 0xBF000000BF000000ull;
+    constexpr uint64_t kTwo23 = 0x4B0000004B000000ull;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        float q0, q1, f0, f1;
+        f2_unpack(NQ[h], q0, q1);
+        f2_unpack(f2_add_rz(f2_mul(f2_fma(NQ[h], kNHalf, kHalf), size), kTwo23), f0, f1);
+        if (!INSIDE) {
+            in[2 * h] = in[2 * h] && fabsf(q0) <= 1.0f;
+            in[2 * h + 1] = in[2 * h + 1] && fabsf(q1) <= 1.0f;
+        }
+        bits[2 * h] = __float_as_uint(f0);
+        bits[2 * h + 1] = __float_as_uint(f1);
     }
 }
 
-// Two views whose T rows y and w are bitwise equal (a stereo pair built as
-// translate(-+ipd/2, 0, 0) * V_head, whose eyes differ in row x only) and whose
-// slots hold the same Wf, Hf and W: y, w, 1/w, the inside test of y and the
-// pixel row are computed once per point, x and the pixel column per view.
-// Every value is the one splat_view computes (same operations, same operands),
-// so both views' words are unchanged.
-template <int PAYLOAD, bool SAFE>
-__device__ __forceinline__ void splat_pair(const MVArgs& a, unsigned long long* zc, const float* sa,
-                                           const float* sb, const Decoded& d, uint32_t valid_mask,
-                                           uint32_t idx0, const uint4& col) {
-    const float4 t0 = reinterpret_cast<const float4*>(sa)[0];
-    const float4 t1 = reinterpret_cast<const float4*>(sa)[1];
-    const float4 t2 = reinterpret_cast<const float4*>(sa)[2];
-    const float4 t3 = reinterpret_cast<const float4*>(sa)[3];
-    const float4 u0 = reinterpret_cast<const float4*>(sb)[0];
-    const float4 u1 = reinterpret_cast<const float4*>(sb)[1];
-    const float4 u2 = reinterpret_cast<const float4*>(sb)[2];
-    const float4 u3 = reinterpret_cast<const float4*>(sb)[3];
-    // slot layout T0 T1 T3 T4 | T5 T7 T8 T9 | T11 T12 T13 T15 | Wf Hf W fb_off
-    const float aT0 = t0.x, aT1 = t0.y, aT3 = t0.z, aT4 = t0.w, aT5 = t1.x, aT7 = t1.y, aT8 = t1.z;
-    const float aT9 = t1.w, aT11 = t2.x, aT12 = t2.y, aT13 = t2.z, aT15 = t2.w;
-    const float bT0 = u0.x, bT4 = u0.w, bT8 = u1.z, bT12 = u2.y;
-    const float Wf = t3.x, Hf = t3.y;
-    const int32_t W = __float_as_int(t3.z);
-    const uint32_t fa = __float_as_uint(t3.w), fb = __float_as_uint(u3.w);
+// merge_pair without branches: with every view's merges in one loop body the
+// selects run as fast as the branches skip (see emit4).
+__device__ __forceinline__ void merge_keys(int a, int b, bool ok[4], const uint32_t tag[4],
+                                           uint32_t wb[4], uint32_t pl[4]) {
+    const bool m = ok[a] && ok[b] && tag[a] == tag[b];
+    const unsigned long long ka = ((unsigned long long)wb[a] << 32) | pl[a];
+    const unsigned long long kb = ((unsigned long long)wb[b] << 32) | pl[b];
+    const bool less = m && kb < ka;
+    wb[a] = less ? wb[b] : wb[a];
+    pl[a] = less ? pl[b] : pl[a];
+    ok[b] = ok[b] && !m;
+}
+
+// Merges the thread's 4 candidates of one view and emits what is left.  The
+// kernel is bound by instruction issue and the L1 data pipe together (76 % each,
+// 40M points); pairs, merges and the unit split took the frame of 200M points
+// and 64 views from 8416 to 6836 us, 40M 2292 -> 1822, one stereo pair of 20M
+// 139 -> 87.  Branching merges and emits measured 6810, but 813 against 730 us
+// on 16 views of 50M (index payload).  Reading the framebuffer word in front of
+// the atomic, all four at once, measured 7190 -> 8490.
+template <int PAYLOAD>
+__device__ __forceinline__ void emit4(const MVArgs& a, unsigned long long* zc, bool ok[4],
+                                      const uint32_t bx[4], const uint32_t row[4], uint32_t off,
+                                      const uint32_t w[4], uint32_t idx0, const uint4& col) {
+    uint32_t tag[4], wb[4], pl[4];
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-        const float x = d.x[j], y = d.y[j], z = d.z[j];
-        const float py = __fmaf_rn(aT9, z, __fmaf_rn(aT5, y, __fmaf_rn(aT1, x, aT13)));
-        const float pw = __fmaf_rn(aT11, z, __fmaf_rn(aT7, y, __fmaf_rn(aT3, x, aT15)));
-        const float rw = SAFE ? rcp_rn_normal(pw) : rcp_rn(pw);
-        const float qy = fmul(py, rw);
-        const bool yin = ((valid_mask >> j) & 1u) && (SAFE || pw > 0.0f) && qy >= -1.0f && qy <= 1.0f;
-        const int32_t row = small_f2i(fmul(__fmaf_rn(qy, 0.5f, 0.5f), Hf)) * W;
-        const uint32_t wbits = __float_as_uint(pw);
+        tag[j] = bx[j] + row[j] + off;
+        wb[j] = w[j];
+        pl[j] = PAYLOAD == CR_PAYLOAD_COLOR ? u4get(col, j) : idx0 + (uint32_t)j;
+    }
+    merge_keys(0, 1, ok, tag, wb, pl);
+    merge_keys(2, 3, ok, tag, wb, pl);
+    merge_keys(0, 2, ok, tag, wb, pl);
+#pragma unroll
+    for (int j = 0; j < 4; j++) emit_mv(a.fbs, zc, ok[j], tag[j], wb[j], pl[j]);
+}
+
+// Projects the 4 decoded points into the w-safe view in slot `sa` (and, with
+// TWO, the view in slot `sb`) and splats them.
+//
+// TWO: two views whose T rows y and w are bitwise equal (a stereo pair built as
+// translate(-+ipd/2, 0, 0) * V_head, whose eyes differ in row x only) and of
+// equal size: y, w, 1/w, the inside test of y and the pixel row are computed
+// once per point, x and the pixel column per view.  Every value is the one the
+// view alone computes (same operations, same operands).
+// INSIDE: every point of the batch is proven to project inside the view(s).
+template <int PAYLOAD, bool TWO, bool INSIDE>
+__device__ __forceinline__ void splat_pairs(const MVArgs& a, unsigned long long* zc, const float* sa,
+                                            const float* sb, const Decoded& d, uint32_t valid_mask,
+                                            uint32_t idx0, const uint4& col) {
+    constexpr uint64_t kOne = 0x3F8000003F800000ull;
+    uint64_t P[2], NR[2], NQ[2];
+    uint32_t wb[4], row[4], bx[4];
+    bool yin[4];
+    project_row(sa, kRowW, d, P);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        NR[h] = f2_neg_rcp_rn_normal(P[h], kOne);
+        float w0, w1;
+        f2_unpack(P[h], w0, w1);
+        wb[2 * h] = __float_as_uint(w0);
+        wb[2 * h + 1] = __float_as_uint(w1);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) yin[j] = (valid_mask >> j) & 1u;
+    const float4 size = *reinterpret_cast<const float4*>(sa + kSize);  // Wf, Hf, W, offset
+    project_row(sa, kRowY, d, P);
+#pragma unroll
+    for (int h = 0; h < 2; h++) NQ[h] = f2_mul(P[h], NR[h]);
+    screen_axis<INSIDE>(NQ, f2_pack(size.y, size.y), yin, row);
+#pragma unroll
+    for (int j = 0; j < 4; j++) row[j] *= __float_as_uint(size.z);
+#pragma unroll
+    for (int e = 0; e < (TWO ? 2 : 1); e++) {
+        const float* sv = e ? sb : sa;
+        const uint32_t off = __float_as_uint(e ? sb[kInts + 1] : size.w);
+        bool ok[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) ok[j] = yin[j];
+        project_row(sv, kRowX, d, P);
+#pragma unroll
+        for (int h = 0; h < 2; h++) NQ[h] = f2_mul(P[h], NR[h]);
+        screen_axis<INSIDE>(NQ, f2_pack(size.x, size.x), ok, bx);
+        emit4<PAYLOAD>(a, zc, ok, bx, row, off, wb, idx0, col);
+    }
+}
+
+// The same for a view whose w range is not proven: one point at a time.
+template <int PAYLOAD>
+__device__ __forceinline__ void splat_scalar(const MVArgs& a, unsigned long long* zc, const float* sv,
+                                             const Decoded& d, uint32_t valid_mask, uint32_t idx0,
+                                             const uint4& col) {
+    BatchCtx c;
+    c.T3 = sv[kRowW]; c.T7 = sv[kRowW + 1]; c.T11 = sv[kRowW + 2]; c.T15 = sv[kRowW + 3];
+    c.T0 = sv[kRowX]; c.T4 = sv[kRowX + 1]; c.T8 = sv[kRowX + 2]; c.T12 = sv[kRowX + 3];
+    c.T1 = sv[kRowY]; c.T5 = sv[kRowY + 1]; c.T9 = sv[kRowY + 2]; c.T13 = sv[kRowY + 3];
+    c.Wf = sv[kSize];
+    c.Hf = sv[kSize + 1];
+    c.W = __float_as_int(sv[kInts]);
+    const uint32_t off = __float_as_uint(sv[kInts + 1]) + pixel_bias(c.W);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        float x[2], y[2], z[2];
+        f2_unpack(d.x[j >> 1], x[0], x[1]);
+        f2_unpack(d.y[j >> 1], y[0], y[1]);
+        f2_unpack(d.z[j >> 1], z[0], z[1]);
+        int32_t pix;
+        uint32_t wbits;
+        const bool ok = project(c, x[j & 1], y[j & 1], z[j & 1], pix, wbits) && ((valid_mask >> j) & 1u);
         const uint32_t payload = (PAYLOAD == CR_PAYLOAD_COLOR) ? u4get(col, j) : idx0 + (uint32_t)j;
-        const float pxa = __fmaf_rn(aT8, z, __fmaf_rn(aT4, y, __fmaf_rn(aT0, x, aT12)));
-        const float qxa = fmul(pxa, rw);
-        const bool oka = yin && qxa >= -1.0f && qxa <= 1.0f;
-        emit_mv(a.fbs, zc, oka, small_f2i(fmul(__fmaf_rn(qxa, 0.5f, 0.5f), Wf)) + row, fa, wbits, payload);
-        const float pxb = __fmaf_rn(bT8, z, __fmaf_rn(bT4, y, __fmaf_rn(bT0, x, bT12)));
-        const float qxb = fmul(pxb, rw);
-        const bool okb = yin && qxb >= -1.0f && qxb <= 1.0f;
-        emit_mv(a.fbs, zc, okb, small_f2i(fmul(__fmaf_rn(qxb, 0.5f, 0.5f), Wf)) + row, fb, wbits, payload);
+        emit_mv(a.fbs, zc, ok, (uint32_t)pix + off, wbits, payload);
     }
 }
 
@@ -285,17 +374,21 @@ __device__ __forceinline__ void mv_raster_items(const MVArgs& a) {
     uint32_t* cursor = a.scratch + (LIST == 0 ? kCursor0 : kCursor2);
     const uint32_t nitems =
         *reinterpret_cast<volatile uint32_t*>(a.scratch + (LIST == 0 ? kItemCount : kItemCount2));
-    if (nitems == 0) return;
+    const WorkSplit ws = split_work<BLOCK>(nitems, gridDim.x, false);
+    if (blockIdx.x >= ws.units) return;
     const uint4* items = reinterpret_cast<const uint4*>(a.scratch + kScratchHead);
     for (int i = threadIdx.x; i < kZCacheSlots; i += BLOCK) s_zc[i] = kZCacheEmpty;
-    if (threadIdx.x == 0) s_item[0] = atomicAdd(cursor, 1u);
+    if (threadIdx.x == 0) s_item[0] = blockIdx.x;
     __syncthreads();
     const bool l0_x12 = (a.quirks & CR_QUIRK_L0_X12) != 0;
     int buf = 0;
     while (true) {
-        const uint32_t wi = s_item[buf];
-        if (wi >= nitems) break;
-        if (threadIdx.x == 0) s_item[buf ^ 1] = atomicAdd(cursor, 1u);
+        const uint32_t unit = s_item[buf];
+        if (unit >= ws.units) break;
+        if (threadIdx.x == 0) s_item[buf ^ 1] = gridDim.x + atomicAdd(cursor, 1u);
+        uint32_t wi;
+        int vb, ve;
+        unit_range(ws, unit, &wi, &vb, &ve);
         const uint4 it = items[LIST == 0 ? (int64_t)wi : a.list_cap - 1 - (int64_t)wi];
         const uint32_t b = it.x, g = it.y, vismask = it.z, levels = it.w;
         const int4* r4 = reinterpret_cast<const int4*>(a.batches + b);
@@ -310,12 +403,18 @@ __device__ __forceinline__ void mv_raster_items(const MVArgs& a) {
             const int s = t / kSlotWords, k = t - s * kSlotWords;
             const int v = (int)g * a.G + s;
             if (((vismask >> s) & 1u) == 0u || v >= a.nviews) continue;
-            float val;
-            if (k < 12) val = a.files[(int64_t)v * a.nfiles + fi].T[k];
-            else if (k == 12) val = (float)a.views[v].W;
-            else if (k == 13) val = (float)a.views[v].H;
-            else if (k == 14) val = __int_as_float(a.views[v].W);
-            else val = __uint_as_float(a.views[v].fb_off);
+            // (T0 T1 T3 | T4 T5 T7 | T8 T9 T11 | T12 T13 T15): column k % 4 of row
+            // w (entry 2), x (0) or y (1)
+            float val = 0.0f;
+            if (k < kSize)
+                val = a.files[(int64_t)v * a.nfiles + fi].T[3 * (k & 3) + (k < kRowX ? 2 : (k < kRowY ? 0 : 1))];
+            else if (k < kInts)
+                val = (float)(k < kSize + 1 ? a.views[v].W : a.views[v].H);
+            else
+            if (k == kInts)
+                val = __int_as_float(a.views[v].W);
+            else if (k == kInts + 1)
+                val = __uint_as_float(a.views[v].fb_off - pixel_bias(a.views[v].W));
             s_view[s][k] = val;
         }
         __syncthreads();
@@ -326,7 +425,7 @@ __device__ __forceinline__ void mv_raster_items(const MVArgs& a) {
         const bool single = LIST == 0 || __popc(classes) == 1;
         const int only = LIST == 0 ? 2 : __ffs(classes) - 1;
         // shared pairs of this item: both views visible, at one level class,
-        // with the same w-range proof
+        // both with a proven w range
         uint32_t pairs = 0;
         if (a.pairs) {
             const uint32_t cand = a.pairs[g] & vismask & (vismask >> 1);
@@ -334,8 +433,8 @@ __device__ __forceinline__ void mv_raster_items(const MVArgs& a) {
                 if (((cand >> s) & 1u) == 0u) continue;
                 const bool same_level =
                     LIST == 0 || level_class((levels >> (3 * s)) & 7u) == level_class((levels >> (3 * s + 3)) & 7u);
-                const bool same_safe = (((levels >> (24 + s)) ^ (levels >> (25 + s))) & 1u) == 0u;
-                if (same_level && same_safe) pairs |= 1u << s;
+                const bool both_safe = ((levels >> (24 + s)) & (levels >> (25 + s)) & 1u) != 0u;
+                if (same_level && both_safe) pairs |= 1u << s;
             }
         }
         const bool need8 = LIST == 1 && (classes & 3u) != 0;
@@ -353,21 +452,23 @@ __device__ __forceinline__ void mv_raster_items(const MVArgs& a) {
         // raster: with firstPoint % 4 != 0 the vectors v % 128 == 0 (the
         // reference's thread 0) are skipped and none past 2559 is read
         const bool uvec4 = head != 0 && (a.quirks & CR_QUIRK_UVEC4_BASE) != 0;
-        const int nv = uvec4 ? min((head + count + 3) >> 2, kPointsPerBatch / 4) : (head + count + 3) >> 2;
+        const int nv = min(ve, uvec4 ? min((head + count + 3) >> 2, kPointsPerBatch / 4)
+                                     : (head + count + 3) >> 2);
         const uint32_t index0 = (uint32_t)(first - head);
+        const bool whole = count == kPointsPerBatch && head == 0;  // every lane's 4 points are the batch's
         const uint4* lo4 = reinterpret_cast<const uint4*>(a.lo) + v0;
         const uint4* md4 = reinterpret_cast<const uint4*>(a.md) + v0;
         const uint4* hi4 = reinterpret_cast<const uint4*>(a.hi) + v0;
         const uint4* co4 = reinterpret_cast<const uint4*>(a.rgba) + v0;
         const uint4 zero = make_uint4(0, 0, 0, 0);
         uint4 n4 = zero, n8 = zero, n12 = zero, ncol = zero;
-        if ((int)threadIdx.x < nv) {
-            n4 = ld_stream(lo4 + threadIdx.x);
-            if (need8) n8 = ld_stream(md4 + threadIdx.x);
-            if (need12) n12 = ld_stream(hi4 + threadIdx.x);
-            if (PAYLOAD == CR_PAYLOAD_COLOR) ncol = ld_stream(co4 + threadIdx.x);
+        if (vb + (int)threadIdx.x < nv) {
+            n4 = ld_stream(lo4 + vb + threadIdx.x);
+            if (need8) n8 = ld_stream(md4 + vb + threadIdx.x);
+            if (need12) n12 = ld_stream(hi4 + vb + threadIdx.x);
+            if (PAYLOAD == CR_PAYLOAD_COLOR) ncol = ld_stream(co4 + vb + threadIdx.x);
         }
-        for (int base = 0; base < nv; base += BLOCK) {
+        for (int base = vb; base < nv; base += BLOCK) {
             const int v = base + (int)threadIdx.x;
             const uint4 w4 = n4, w8 = n8, w12 = n12, col = ncol;
             const int vn = v + BLOCK;
@@ -392,19 +493,21 @@ __device__ __forceinline__ void mv_raster_items(const MVArgs& a) {
                 if (LIST == 1 && !single)
                     decode4(level_class((levels >> (3 * s)) & 7u), w4, w8, w12, mnx, mny, mnz, sc,
                             l0_x12, d);
-                // views whose w range is proven safe skip the reciprocal's range
-                // test (measured 12 % faster on the 64-view frame)
                 const bool safe = (levels >> (24 + s)) & 1u;
+                const bool in0 = whole && ((levels >> (3 * s)) & 7u) >= 2u + kLevelInside;
                 if ((pairs >> s) & 1u) {
-                    if (safe)
-                        splat_pair<PAYLOAD, true>(a, s_zc, s_view[s], s_view[s + 1], d, valid_mask, idx0, col);
+                    const bool in1 = ((levels >> (3 * s + 3)) & 7u) >= 2u + kLevelInside;
+                    if (in0 && in1)
+                        splat_pairs<PAYLOAD, true, true>(a, s_zc, s_view[s], s_view[s + 1], d, 15u, idx0, col);
                     else
-                        splat_pair<PAYLOAD, false>(a, s_zc, s_view[s], s_view[s + 1], d, valid_mask, idx0, col);
+                        splat_pairs<PAYLOAD, true, false>(a, s_zc, s_view[s], s_view[s + 1], d, valid_mask, idx0, col);
                     s++;
+                } else if (in0) {
+                    splat_pairs<PAYLOAD, false, true>(a, s_zc, s_view[s], nullptr, d, 15u, idx0, col);
                 } else if (safe) {
-                    splat_view<PAYLOAD, true>(a, s_zc, s_view[s], d, valid_mask, idx0, col);
+                    splat_pairs<PAYLOAD, false, false>(a, s_zc, s_view[s], nullptr, d, valid_mask, idx0, col);
                 } else {
-                    splat_view<PAYLOAD, false>(a, s_zc, s_view[s], d, valid_mask, idx0, col);
+                    splat_scalar<PAYLOAD>(a, s_zc, s_view[s], d, valid_mask, idx0, col);
                 }
             }
         }
@@ -417,35 +520,58 @@ __device__ __forceinline__ void mv_raster_items(const MVArgs& a) {
 // (programmatic dependent launch); every list-0 CTA waits for the list-1 grid
 // before it exits, so the resolve that follows sees both lists' writes.
 template <int PAYLOAD, int BLOCK, int LIST>
-__global__ void __launch_bounds__(BLOCK) k_mv_raster(MVArgs a) {
+__global__ void __launch_bounds__(BLOCK, (LIST == 0 ? 8 : 5) * 128 / BLOCK) k_mv_raster(MVArgs a) {
     if (LIST == 1) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     mv_raster_items<PAYLOAD, BLOCK, LIST>(a);
     if (LIST == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-__global__ void k_mv_resolve(const MVView* __restrict__ views, unsigned long long* fbs,
-                             uint32_t* images, const uint32_t* __restrict__ rgba,
-                             int64_t rgba_words, int32_t payload, int32_t clear_after,
-                             unsigned long long clear) {
-    const MVView vw = views[blockIdx.y];
-    const int64_t P = (int64_t)vw.W * vw.H, tail = (int64_t)vw.W + 1;
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    unsigned long long* fb = fbs + vw.fb_off;
-    if (t < P) {
-        const unsigned long long w = fb[t];
-        const float dpt = __uint_as_float((uint32_t)(w >> 32));
-        const bool valid = dpt > 0.0f && dpt < 1000000.0f;  // resolve.cs:124
-        uint32_t out;
-        if (payload == CR_PAYLOAD_COLOR) {
-            out = valid ? (uint32_t)w : kBackground;
-        } else {
-            const uint32_t id = valid ? (uint32_t)w : 0u;
-            out = (id == 0u || id >= rgba_words) ? kBackground : __ldg(rgba + id);
+// Bound by its bytes (20 per pixel): 82M pixels of 64 views take 252 us, 6.5 TB/s.
+// One thread per pixel on a grid of the largest view for every view launched
+// 576,384 CTAs, with one load in flight per thread or none, and took 430 us.
+// Grid y: views; grid x strides over a view's pixels in tiles of kResolvePix
+// pixels per thread, whose loads are all in flight before the first is used.
+constexpr int kResolvePix = 4;
+__global__ void __launch_bounds__(256) k_mv_resolve(const MVView* __restrict__ views,
+                                                    unsigned long long* fbs, uint32_t* images,
+                                                    const uint32_t* __restrict__ rgba,
+                                                    int64_t rgba_words, int32_t payload,
+                                                    int32_t clear_after, unsigned long long clear) {
+    const int32_t W = views[blockIdx.y].W, H = views[blockIdx.y].H;
+    unsigned long long* fb = fbs + views[blockIdx.y].fb_off;
+    uint32_t* image = images + views[blockIdx.y].img_off;
+    const uint32_t P = (uint32_t)W * (uint32_t)H;  // below 2^31
+    const uint32_t tile = 256u * kResolvePix;
+    for (uint32_t base = blockIdx.x * tile; base < P; base += gridDim.x * tile) {
+        unsigned long long w[kResolvePix];
+#pragma unroll
+        for (int k = 0; k < kResolvePix; k++) {
+            const uint32_t t = base + threadIdx.x + 256u * k;
+            w[k] = t < P ? fb[t] : 0ull;
         }
-        images[vw.img_off + t] = out;
-        if (clear_after) fb[t] = clear;
+        uint32_t out[kResolvePix];
+#pragma unroll
+        for (int k = 0; k < kResolvePix; k++) {
+            const float dpt = __uint_as_float((uint32_t)(w[k] >> 32));
+            const bool valid = dpt > 0.0f && dpt < 1000000.0f;  // resolve.cs:124
+            if (payload == CR_PAYLOAD_COLOR) {
+                out[k] = valid ? (uint32_t)w[k] : kBackground;
+            } else {
+                const uint32_t id = valid ? (uint32_t)w[k] : 0u;
+                out[k] = (id == 0u || id >= rgba_words) ? kBackground : __ldg(rgba + id);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kResolvePix; k++) {
+            const uint32_t t = base + threadIdx.x + 256u * k;
+            if (t >= P) break;
+            image[t] = out[k];
+            if (clear_after) fb[t] = clear;
+        }
     }
-    if (clear_after && t < tail) fb[P + t] = clear;
+    if (!clear_after) return;
+    for (uint32_t t = blockIdx.x * 256u + threadIdx.x; t <= (uint32_t)W; t += gridDim.x * 256u)
+        fb[P + t] = clear;  // the guard tail of W + 1 words
 }
 
 __global__ void k_mv_fill(unsigned long long* p, int64_t n, unsigned long long v) {
@@ -602,7 +728,10 @@ cr_status mv_enqueue(const MVFrame& f, void* stream, const char** what) {
         if (e != cudaSuccess) return fail("raster launch");
     }
     if (f.resolve) {
-        const unsigned gx = (unsigned)((words + 255) / 256);
+        // eight waves of resident CTAs over all views, none past the largest view
+        const int64_t tiles = (words + 256 * kResolvePix - 1) / (256 * kResolvePix);
+        const int64_t share = std::max<int64_t>((int64_t)f.num_sms * 64 / f.nviews, 1);
+        const unsigned gx = (unsigned)std::min(tiles, share);
         if (launch_k(k_mv_resolve, dim3(gx, (unsigned)f.nviews), 256, st, f.d_views,
                      reinterpret_cast<unsigned long long*>(f.fbs), f.images, f.ci.rgba, f.ci.capacity,
                      f.payload, f.clear_after, f.clear_value) != 0)

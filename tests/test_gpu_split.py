@@ -1,10 +1,12 @@
-"""The unit split of the batched kernels (whole batches first, the last item
-per CTA in parts): item counts around every switch of the rule, against the
-oracle, bit for bit."""
+"""The unit split of the batched and multi-view kernels (whole batches first, the
+last item per CTA in parts): item counts around every switch of the rule,
+against the oracle, bit for bit."""
 import numpy as np
 import pytest
 
 from compute_rasterizer_gb300 import _lib as L
+from compute_rasterizer_gb300 import default_params, make_view
+from compute_rasterizer_gb300.multiview import MultiView
 from helpers import QUIRKS, cameras, encoded, first_diff, gpu_raw, oracle_frame
 from oracle import oracle as O
 
@@ -50,5 +52,35 @@ def test_item_counts(ctx, cloud_310, items, ctas, block):
         assert np.array_equal(fb.read(L.FB_DEPTH), depth)
         assert np.array_equal(fb.read(L.FB_ACCUM), accum)
         fb.close()
+    finally:
+        cloud.set_loaded()
+
+
+# Two views per group: an item per batch and group.  The third view makes a
+# second group of one view, so counts are twice the batches.
+@pytest.mark.parametrize("block", [64, 128, 256])
+@pytest.mark.parametrize("batches", [1, 15, 16, 30, 31, 76, 77, 310])
+def test_multiview_item_counts(ctx, cloud_310, batches, block):
+    cl, cloud = cloud_310
+    points = min(cl["n"], batches * L.POINTS_PER_BATCH)
+    cloud.set_loaded(points, batches)
+    cams = [cameras(cl, 97, 61)[k] for k in ("far", "corner", "mid")]
+    params = default_params(L.METHOD_LOOP_LAS, frustum_culling=0, views_per_group=2, ctas_per_sm=1,
+                            block_threads=block, clear_after=0)
+    try:
+        mv = MultiView(ctx, cloud, [(c[2], c[3]) for c in cams], params)
+        mv.set_views([make_view(*c) for c in cams])
+        mv.clear()
+        mv.render()
+        ctx.sync()
+        for i, cam in enumerate(cams):
+            fr = oracle_frame(cam, cl["box_min"][None], QUIRKS[L.METHOD_LOOP_LAS], culling=0)
+            want = O.raster_batched(fr, cl["batches"][:batches], points, cl["lo"], cl["md"],
+                                    cl["hi"], cl["rgba"])
+            got = mv.read(i, L.FB_WORDS)
+            assert np.array_equal(got, want), (i, first_diff(got, want))
+            img = O.resolve_index(cam[2], cam[3], want, cl["rgba"])
+            assert np.array_equal(mv.read(i, L.FB_IMAGE), img), i
+        mv.close()
     finally:
         cloud.set_loaded()
