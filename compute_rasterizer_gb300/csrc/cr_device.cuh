@@ -269,17 +269,20 @@ __device__ __forceinline__ WorkSplit split_work(uint32_t nitems, uint32_t ctas, 
 }
 
 // The list item of a unit and its range of vectors.
-__device__ __forceinline__ void unit_range(const WorkSplit& ws, uint32_t unit, uint32_t* item, int* vb,
-                                           int* ve) {
-    *item = unit;
-    *vb = 0;
-    *ve = kAllVectors;
-    if (unit < ws.whole) return;
-    const uint32_t k = (unit - ws.whole) / ws.parts, part = (unit - ws.whole) - k * ws.parts;
-    *item = ws.whole + k;
-    *vb = (int)part * ws.part_vectors;
-    // the last part of an unaligned batch takes its extra vector too
-    if (part + 1 != ws.parts) *ve = *vb + ws.part_vectors;
+struct Unit {
+    uint32_t item;
+    int vb, ve;
+};
+__device__ __forceinline__ Unit unit_range(const WorkSplit& ws, uint32_t unit) {
+    Unit u{unit, 0, kAllVectors};
+    if (unit >= ws.whole) {
+        u.item = ws.whole + (unit - ws.whole) / ws.parts;
+        const uint32_t part = (unit - ws.whole) % ws.parts;
+        u.vb = (int)part * ws.part_vectors;
+        // the last part of an unaligned batch takes its extra vector too
+        u.ve = part + 1 == ws.parts ? kAllVectors : u.vb + ws.part_vectors;
+    }
+    return u;
 }
 
 struct BatchCtx {

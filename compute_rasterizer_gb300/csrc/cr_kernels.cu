@@ -469,9 +469,9 @@ __global__ void __launch_bounds__(BLOCK, (kMinBlocks<MODE, BLOCK, LIST, MANY && 
             const uint32_t unit = s_item[buf];
             if (unit >= ws.units) break;
             if (threadIdx.x == 0) s_item[buf ^ 1] = gridDim.x + atomicAdd(cursor, 1u);
-            uint32_t wi;
-            int vb, ve;
-            unit_range(ws, unit, &wi, &vb, &ve);
+            const Unit u = unit_range(ws, unit);
+            const uint32_t wi = u.item;
+            const int vb = u.vb, ve = u.ve;
             const uint32_t item =
                 bl.scratch[kScratchHead + (LIST == 0 ? (int64_t)wi : bl.list_cap - 1 - (int64_t)wi)];
             const uint32_t b = item & (bl.node_slices ? kItemNodeMask : kItemBatchMask);

@@ -386,9 +386,9 @@ __device__ __forceinline__ void mv_raster_items(const MVArgs& a) {
         const uint32_t unit = s_item[buf];
         if (unit >= ws.units) break;
         if (threadIdx.x == 0) s_item[buf ^ 1] = gridDim.x + atomicAdd(cursor, 1u);
-        uint32_t wi;
-        int vb, ve;
-        unit_range(ws, unit, &wi, &vb, &ve);
+        const Unit u = unit_range(ws, unit);
+        const uint32_t wi = u.item;
+        const int vb = u.vb, ve = u.ve;
         const uint4 it = items[LIST == 0 ? (int64_t)wi : a.list_cap - 1 - (int64_t)wi];
         const uint32_t b = it.x, g = it.y, vismask = it.z, levels = it.w;
         const int4* r4 = reinterpret_cast<const int4*>(a.batches + b);
