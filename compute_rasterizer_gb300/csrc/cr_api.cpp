@@ -33,6 +33,11 @@ struct cr_ctx {
     int64_t last_dispatched = 0;  // batch records the last cull looked at
     int64_t last_list_cap = 0;    // words of its item-list region
     bool last_node_slices = false;
+    bool last_resolved = false;
+    // whether the next frame finds the counters at zero: a frame's resolve
+    // leaves them so; one without a resolve, or that failed on the way, does not
+    bool counters_zero = false;
+    bool captured = false;  // a frame was captured into a graph
     std::vector<cr_frame_events> timing;  // GLTimerQueries-style event pairs
     int32_t timing_used = 0;
     std::string last_error;
@@ -172,8 +177,12 @@ cr_status ensure_scratch(cr_ctx* ctx, int64_t items) {
     CR_CUDA(ctx, cudaMalloc(&ctx->scratch, words * 4), "scratch allocation");
     CR_CUDA(ctx, cudaMemset(ctx->scratch, 0, words * 4), "scratch clear");
     ctx->scratch_words = words;
+    ctx->counters_zero = false;  // cleared on another stream than the frame's, perhaps
     return CR_OK;
 }
+
+// Where a frame's resolve leaves its two item counts, past the list region.
+uint32_t* frame_counts(const cr_ctx* ctx) { return ctx->scratch + ctx->scratch_words - 2; }
 
 constexpr int kNumMethods = 7;
 const char* kNames[kNumMethods] = {"loop_las",       "loop_las_prefetch", "loop_las_hqs",
@@ -724,13 +733,14 @@ cr_status cr_fb_read(cr_ctx* ctx, const cr_fb* f, int32_t what, void* dst, int64
 
 // ---- rendering ------------------------------------------------------------------
 
-cr_status cr_resolve(cr_ctx* ctx, const cr_cloud* cloud, const cr_render_params* p, cr_fb* fb,
-                     void* stream) {
-    if (!ctx || !p || !fb) return CR_ERR_INVALID_ARG;
+// scratch, counts: see launch_resolve_index.
+static cr_status resolve_into(cr_ctx* ctx, const cr_cloud* cloud, const cr_render_params* p, cr_fb* fb,
+                              void* stream, uint32_t* scratch, uint32_t* counts) {
     int rc;
     if (p->method == CR_METHOD_LOOP_LAS_HQS) {
         if (fb->kind != CR_FB_HQS) return fail(ctx, CR_ERR_INVALID_ARG, "HQS needs an HQS fb%s", "");
-        rc = launch_resolve_hqs(fb->W, fb->H, fb->depth, fb->accum, fb->image, p->clear_after, stream);
+        rc = launch_resolve_hqs(fb->W, fb->H, fb->depth, fb->accum, fb->image, p->clear_after, stream,
+                                scratch, counts);
     } else {
         if (fb->kind != CR_FB_U64) return fail(ctx, CR_ERR_INVALID_ARG, "method needs a u64 fb%s", "");
         if (plain_method(p->method)) {
@@ -743,19 +753,25 @@ cr_status cr_resolve(cr_ctx* ctx, const cr_cloud* cloud, const cr_render_params*
             const int tiles = (quirks & CR_QUIRK_RESOLVE_TILES) ? 1 : 0;
             if (p->payload == CR_PAYLOAD_COLOR && !tiles) {
                 rc = launch_resolve_color(fb->W, fb->H, fb->fb, fb->image, p->clear_after, p->clear_value,
-                                          stream);
+                                          stream, scratch, counts);
             } else if (p->payload == CR_PAYLOAD_COLOR) {
                 return fail(ctx, CR_ERR_UNSUPPORTED, "the tiled resolve reads the index payload%s", "");
             } else {
                 if (!cloud || !cloud->rgba)
                     return fail(ctx, CR_ERR_INVALID_ARG, "index payload resolve needs the color stream%s", "");
                 rc = launch_resolve_index(fb->W, fb->H, fb->fb, cloud->rgba, cloud->capacity, fb->image,
-                                          p->clear_after, p->clear_value, stream, tiles);
+                                          p->clear_after, p->clear_value, stream, tiles, scratch, counts);
             }
         }
     }
     if (rc != 0) return fail(ctx, CR_ERR_CUDA, "resolve launch failed%s", "");
     return CR_OK;
+}
+
+cr_status cr_resolve(cr_ctx* ctx, const cr_cloud* cloud, const cr_render_params* p, cr_fb* fb,
+                     void* stream) {
+    if (!ctx || !p || !fb) return CR_ERR_INVALID_ARG;
+    return resolve_into(ctx, cloud, p, fb, stream, nullptr, nullptr);
 }
 
 cr_status cr_render(cr_ctx* ctx, const cr_cloud* cloud, const cr_view* view,
@@ -846,8 +862,17 @@ cr_status cr_render(cr_ctx* ctx, const cr_cloud* cloud, const cr_view* view,
     ctx->last_dispatched = nb;
     ctx->last_list_cap = list_cap;
     ctx->last_node_slices = slices;
+    ctx->last_resolved = p->resolve != 0;
 
-    CR_CUDA(ctx, cudaMemsetAsync(ctx->scratch, 0, kCounterWords * 4, st), "counter reset");
+    // a captured frame runs at times this host code does not see, so it, and every
+    // frame after it, zeroes the counters itself
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (st != nullptr && st != cudaStreamLegacy &&
+        (cudaStreamIsCapturing(st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone))
+        ctx->captured = true;
+    if (!ctx->counters_zero || ctx->captured)
+        CR_CUDA(ctx, cudaMemsetAsync(ctx->scratch, 0, kCounterWords * 4, st), "counter reset");
+    ctx->counters_zero = false;
     if (launch_cull(vp, cloud->batches, nb, cloud->capacity, quirks, ctx->scratch, stream, list_cap,
                     slices ? 1 : 0) != 0)
         return fail(ctx, CR_ERR_CUDA, "cull launch failed%s", "");
@@ -888,8 +913,9 @@ cr_status cr_render(cr_ctx* ctx, const cr_cloud* cloud, const cr_view* view,
         mark(2 + pass, pass == 0 ? CR_STAGE_RASTER : CR_STAGE_HQS_COLOR);
     }
     if (p->resolve) {
-        s = cr_resolve(ctx, cloud, p, fb, stream);
+        s = resolve_into(ctx, cloud, p, fb, stream, ctx->scratch, frame_counts(ctx));
         if (s != CR_OK) return s;
+        ctx->counters_zero = true;
     }
     mark(4, p->resolve ? CR_STAGE_RESOLVE : -1);
     return CR_OK;
@@ -900,9 +926,12 @@ cr_status cr_last_frame_stats(cr_ctx* ctx, const cr_cloud* cloud, const cr_rende
     if (!ctx || !cloud || !p || !out || cloud->plain) return CR_ERR_INVALID_ARG;
     std::memset(out, 0, sizeof(*out));
     CR_CUDA(ctx, cudaDeviceSynchronize(), "synchronize");
+    // counts of a frame without a resolve are still where the cull counted
     uint32_t counts[kCounterWords] = {};
-    CR_CUDA(ctx, cudaMemcpy(counts, ctx->scratch, sizeof(counts), cudaMemcpyDeviceToHost), "count read");
-    const uint32_t n_front = counts[kItemCount], n_back = counts[kItemCount2];
+    CR_CUDA(ctx, cudaMemcpy(counts, ctx->last_resolved ? frame_counts(ctx) : ctx->scratch,
+                            (ctx->last_resolved ? 2 : kCounterWords) * 4, cudaMemcpyDeviceToHost),
+            "count read");
+    const uint32_t n_front = counts[kItemCount], n_back = counts[ctx->last_resolved ? 1 : kItemCount2];
     const uint32_t count = n_front + n_back;
     std::vector<uint32_t> items(count);
     if (n_front)

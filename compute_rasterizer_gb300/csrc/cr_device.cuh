@@ -24,6 +24,31 @@ int launch_k(void (*k)(KArgs...), dim3 grid, dim3 block, cudaStream_t s, Args&&.
     return cudaLaunchKernelEx(&cfg, k, static_cast<Args&&>(args)...) == cudaSuccess ? 0 : -1;
 }
 
+// The same as a programmatic dependent of the stream's previous kernel: the grid
+// may be resident before that one has finished, so every thread of `k` calls
+// grid_wait() before it touches memory.
+template <typename... KArgs, typename... Args>
+int launch_dep(void (*k)(KArgs...), dim3 grid, dim3 block, cudaStream_t s, Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k, static_cast<Args&&>(args)...) == cudaSuccess ? 0 : -1;
+}
+
+// Waits until the grids this one depends on have finished and their writes are
+// visible (at once when it was launched without a dependence).
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets the stream's next dependent grid start once every CTA has called this.
+__device__ __forceinline__ void grid_release() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 constexpr uint32_t kFull = 0xFFFFFFFFu;
 constexpr uint32_t kNoPixel = 0xFFFFFFFFu;
 

@@ -16,25 +16,45 @@
 
 namespace cr {
 
-// glm operator*(mat4, mat4): column c = A[0]*B[c][0] + A[1]*B[c][1] + A[2]*B[c][2] + A[3]*B[c][3]
+// glm operator*(mat4, mat4): column c = A[0]*B[c][0] + A[1]*B[c][1] + A[2]*B[c][2] + A[3]*B[c][3];
+// one entry, from B's column.
+template <typename T>
+__host__ __device__ inline T mat_entry(const T* a, const T* b_col, int row) {
+    T s = a[row] * b_col[0];
+    s = s + a[4 + row] * b_col[1];
+    s = s + a[8 + row] * b_col[2];
+    s = s + a[12 + row] * b_col[3];
+    return s;
+}
+
 template <typename T>
 __host__ __device__ inline void mat_mul(const T* a, const T* b, T* out) {
     T r[16];
-    for (int c = 0; c < 4; c++) {
-        for (int row = 0; row < 4; row++) {
-            T s = a[row] * b[c * 4];
-            s = s + a[4 + row] * b[c * 4 + 1];
-            s = s + a[8 + row] * b[c * 4 + 2];
-            s = s + a[12 + row] * b[c * 4 + 3];
-            r[c * 4 + row] = s;
-        }
-    }
+    for (int c = 0; c < 4; c++)
+        for (int row = 0; row < 4; row++) r[c * 4 + row] = mat_entry(a, b + 4 * c, row);
     for (int i = 0; i < 16; i++) out[i] = r[i];
 }
 
-// render.cs:134-174: planes from the rows of transformFrustum, normalised.
+// render.cs:134-142: one plane from its row combination, normalised.
 // literal (CR_QUIRK_LITERAL_ARITH): `vec3(x, y, z) / nLength` divides each
 // component instead of multiplying by one reciprocal.
+__host__ __device__ inline void frustum_plane(const float* p, float* plane, bool literal) {
+    const float len = sqrtf((p[0] * p[0] + p[1] * p[1]) + p[2] * p[2]);
+    // render.cs:139-140: vec3 / length is one reciprocal, w / length a division
+    if (literal) {
+        plane[0] = p[0] / len;
+        plane[1] = p[1] / len;
+        plane[2] = p[2] / len;
+    } else {
+        const float inv = 1.0f / len;
+        plane[0] = p[0] * inv;
+        plane[1] = p[1] * inv;
+        plane[2] = p[2] * inv;
+    }
+    plane[3] = p[3] / len;
+}
+
+// render.cs:134-174: planes from the rows of transformFrustum.
 __host__ __device__ inline void frustum_planes(const float* m, float* planes, bool literal = false) {
     const float comb[6][4] = {
         {m[3] - m[0], m[7] - m[4], m[11] - m[8], m[15] - m[12]},
@@ -44,22 +64,7 @@ __host__ __device__ inline void frustum_planes(const float* m, float* planes, bo
         {m[3] - m[2], m[7] - m[6], m[11] - m[10], m[15] - m[14]},
         {m[3] + m[2], m[7] + m[6], m[11] + m[10], m[15] + m[14]},
     };
-    for (int i = 0; i < 6; i++) {
-        const float* p = comb[i];
-        const float len = sqrtf((p[0] * p[0] + p[1] * p[1]) + p[2] * p[2]);
-        // render.cs:139-140: vec3 / length is one reciprocal, w / length a division
-        if (literal) {
-            planes[4 * i + 0] = p[0] / len;
-            planes[4 * i + 1] = p[1] / len;
-            planes[4 * i + 2] = p[2] / len;
-        } else {
-            const float inv = 1.0f / len;
-            planes[4 * i + 0] = p[0] * inv;
-            planes[4 * i + 1] = p[1] * inv;
-            planes[4 * i + 2] = p[2] * inv;
-        }
-        planes[4 * i + 3] = p[3] / len;
-    }
+    for (int i = 0; i < 6; i++) frustum_plane(comb[i], planes + 4 * i, literal);
 }
 
 // compute_loop_las.h:166-200 for one file: transform = mat4(proj * view *

@@ -153,18 +153,23 @@ int launch_batched(const ViewParams& vp, const BatchedLaunch& bl, int block, int
 // literal: CR_QUIRK_LITERAL_ARITH
 int launch_plain(const float T[16], int32_t W, int32_t H, const cr_vertex* v, int64_t n,
                  uint64_t* fb, int grid, int variant, void* stream, int literal = 0);
-// tiles: CR_QUIRK_RESOLVE_TILES (image words outside full 16x16 tiles kept)
+// tiles: CR_QUIRK_RESOLVE_TILES (image words outside full 16x16 tiles kept).
+// scratch (the batched resolves): zero its counters, their two item counts kept
+// in counts[0], counts[1]
 int launch_resolve_index(int32_t W, int32_t H, uint64_t* fb, const uint32_t* rgba,
                          int64_t rgba_words, uint32_t* image, int clear_after, uint64_t clear,
-                         void* stream, int tiles = 0);
+                         void* stream, int tiles = 0, uint32_t* scratch = nullptr,
+                         uint32_t* counts = nullptr);
 int launch_resolve_color(int32_t W, int32_t H, uint64_t* fb, uint32_t* image, int clear_after,
-                         uint64_t clear, void* stream);
+                         uint64_t clear, void* stream, uint32_t* scratch = nullptr,
+                         uint32_t* counts = nullptr);
 // tiles: CR_QUIRK_RESOLVE_TILES; zero_rule: ucol == 0 resolves to opaque black
 // (early-z, early-z & reduce; not dedup)
 int launch_resolve_plain(int32_t W, int32_t H, uint64_t* fb, uint32_t* image, int clear_after,
                          uint64_t clear, int tiles, int zero_rule, void* stream);
 int launch_resolve_hqs(int32_t W, int32_t H, uint32_t* depth, uint64_t* accum, uint32_t* image,
-                       int clear_after, void* stream);
+                       int clear_after, void* stream, uint32_t* scratch = nullptr,
+                       uint32_t* counts = nullptr);
 int launch_fill_u64(uint64_t* p, int64_t n, uint64_t v, void* stream);
 int launch_fill_u32(uint32_t* p, int64_t n, uint32_t v, void* stream);
 // rcp_rn against __frcp_rn over every float; counts into bad[0], the lowest

@@ -44,22 +44,67 @@ namespace {
 
 // ---- per-file records of one view (clouds with more than kInlineFiles files)
 
-constexpr int kFilesPerLaunch = 1024;
+// The chunk travels by value in the kernel parameters; the small one keeps them
+// short for the usual cloud.
+constexpr int kFilesPerLaunch = 1024, kFilesSmall = 64;
+template <int N>
 struct FileChunk {
-    double view[16], proj[16];
+    double pv[16], view[16];  // proj * view; with float_uniforms the float product's values
     int32_t first, count, float_uniforms, literal;
-    double box_min[3 * kFilesPerLaunch];
+    double box_min[3 * N];
 };
-static_assert(sizeof(FileChunk) < 32000, "kernel parameters are limited to 32 KB");
+static_assert(sizeof(FileChunk<kFilesPerLaunch>) < 32000, "kernel parameters are limited to 32 KB");
 
-__global__ void __launch_bounds__(128) k_file_records(const __grid_constant__ FileChunk c,
+// file_record() / file_record_float() with one matrix entry per thread, 16
+// threads per file: the same operations on the same operands (proj * view, which
+// every file shares, comes from the host).  One file per thread left one warp a
+// serial chain of 224 double operations: 24 files 10.7 us, now 3.3.
+template <int N>
+__global__ void __launch_bounds__(128) k_file_records(const __grid_constant__ FileChunk<N> c,
                                                       FileRec* __restrict__ out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.count) return;
-    FileRec r;
-    if (c.float_uniforms) file_record_float(c.view, c.proj, &c.box_min[3 * i], &r, c.literal != 0);
-    else file_record(c.view, c.proj, &c.box_min[3 * i], &r, c.literal != 0);
-    out[c.first + i] = r;
+    grid_wait();
+    __shared__ float s_T[8][16];
+    const int slot = threadIdx.x >> 4, e = threadIdx.x & 15, col = e >> 2, row = e & 3;
+    const int i = blockIdx.x * 8 + slot;
+    const bool act = i < c.count;
+    if (act) {
+        // column `col` of translate(boxMin)
+        double w[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+        for (int k = 0; k < 4; k++) w[k] = col == 3 ? (k < 3 ? c.box_min[3 * i + k] : 1.0) : (k == col ? 1.0 : 0.0);
+        float fw[4], fview[16];
+#pragma unroll
+        for (int k = 0; k < 4; k++) fw[k] = (float)w[k];
+#pragma unroll
+        for (int k = 0; k < 16; k++) fview[k] = (float)c.view[k];
+        float t;
+        if (c.float_uniforms) {
+            float fpv[16];
+#pragma unroll
+            for (int k = 0; k < 16; k++) fpv[k] = (float)c.pv[k];
+            t = mat_entry(fpv, fw, row);
+        } else {
+            t = (float)mat_entry(c.pv, w, row);
+        }
+        s_T[slot][e] = t;
+        out[c.first + i].T[e] = t;
+        out[c.first + i].VW[e] = mat_entry(fview, fw, row);
+    }
+    __syncwarp();
+    if (act && e < 6) {
+        // frustum_planes' row combinations: row 3 -, +, +, -, -, + row 0, 0, 1, 1, 2, 2
+        const float* m = s_T[slot];
+        const bool plus = e == 1 || e == 2 || e == 5;
+        float comb[4], plane[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const float a = m[4 * k + 3], b = m[4 * k + (e >> 1)];
+            comb[k] = plus ? a + b : a - b;
+        }
+        frustum_plane(comb, plane, c.literal != 0);
+#pragma unroll
+        for (int k = 0; k < 4; k++) out[c.first + i].planes[4 * e + k] = plane[k];
+    }
 }
 
 // The record of file `fi`: kernel parameters for the first kInlineFiles files,
@@ -83,6 +128,7 @@ __global__ void __launch_bounds__(256) k_cull(const __grid_constant__ ViewParams
                                               int64_t capacity, int32_t quirks,
                                               uint32_t* __restrict__ scratch, int64_t list_cap,
                                               int32_t node_slices) {
+    grid_wait();
     int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     bool keep = false;
     uint32_t item = 0, slices = 1;
@@ -439,8 +485,14 @@ constexpr int kMinBlocks = MODE != kModeHqsColor || UNCAPPED ? 0 : (LIST == 0 ? 
 // LIST 0: the 10-bit items (front of the list region), LIST 1: the 20/30-bit
 // items (back of the region).  Each list runs in its own instance, so the
 // common 10-bit instance carries no wider decode state (fewer registers).
-// List 1 is launched first and lets the list-0 grid start at once
-// (programmatic dependent launch); every list-0 CTA waits for the list-1 grid
+// The frame's grids are programmatic dependents of one another, so a grid's
+// launch runs behind its predecessor's work (with the counter reset in the
+// resolve and the parallel file records: 50k points 21.3 -> 14.7 us, octree of 2M
+// 41.2 -> 34.8, 24 files 83.8 -> 63.0, 100M flight of 5 frames 840 -> 796).  Only
+// list 1 releases its dependent early: a release at the top of list 0, the cull
+// or the resolves measured level on small frames and slowed HQS 300M from 1442
+// to 1742 us, the waiting CTAs taking room from the running ones.  List 1 waits for the cull, then
+// lets the list-0 grid start at once; every list-0 CTA waits for the list-1 grid
 // before it exits, so work that follows on the stream sees both lists' writes.
 // MANY: the cloud has more than kInlineFiles files, whose records are read
 // from vp.dfiles (a separate instance, so the common case's code is untouched).
@@ -450,7 +502,10 @@ constexpr int kMinBlocks = MODE != kModeHqsColor || UNCAPPED ? 0 : (LIST == 0 ? 
 template <int MODE, int PAYLOAD, int BLOCK, int LIST, bool MANY, bool LIT = false>
 __global__ void __launch_bounds__(BLOCK, (kMinBlocks<MODE, BLOCK, LIST, MANY && LIT>))
     k_batched(ViewParams vp, BatchedLaunch bl, PairParams pp) {
-    if (LIST == 1) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (LIST == 1) {
+        grid_wait();
+        grid_release();
+    }
     __shared__ uint32_t s_item[2];
     __shared__ unsigned long long s_zc[MODE == kModeHqsColor ? 1 : kZCacheSlots];
     uint32_t* cursor = bl.scratch + (LIST == 0 ? (MODE == kModeHqsColor ? kCursor1 : kCursor0)
@@ -472,8 +527,8 @@ __global__ void __launch_bounds__(BLOCK, (kMinBlocks<MODE, BLOCK, LIST, MANY && 
             const Unit u = unit_range(ws, unit);
             const uint32_t wi = u.item;
             const int vb = u.vb, ve = u.ve;
-            const uint32_t item =
-                bl.scratch[kScratchHead + (LIST == 0 ? (int64_t)wi : bl.list_cap - 1 - (int64_t)wi)];
+            const uint32_t item = __ldcg(
+                bl.scratch + kScratchHead + (LIST == 0 ? (int64_t)wi : bl.list_cap - 1 - (int64_t)wi));
             const uint32_t b = item & (bl.node_slices ? kItemNodeMask : kItemBatchMask);
             const int level = (int)(item >> 29);  // levels 2-4 + kLevelInside: inside the view
 
@@ -533,7 +588,7 @@ __global__ void __launch_bounds__(BLOCK, (kMinBlocks<MODE, BLOCK, LIST, MANY && 
             buf ^= 1;
         }
     }
-    if (LIST == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (LIST == 0) grid_wait();
 }
 
 // ---- plain 16 B/point path --------------------------------------------------
@@ -555,6 +610,7 @@ struct PlainParams {
 template <int BLOCK, int VARIANT, bool LIT = false>
 __global__ void __launch_bounds__(BLOCK) k_plain(PlainParams pp, const uint4* __restrict__ v,
                                                  int64_t n, uint64_t* __restrict__ fb) {
+    grid_wait();
     BatchCtx c;
     c.T0 = pp.T[0]; c.T1 = pp.T[1]; c.T3 = pp.T[3];
     c.T4 = pp.T[4]; c.T5 = pp.T[5]; c.T7 = pp.T[7];
@@ -639,6 +695,17 @@ __global__ void __launch_bounds__(BLOCK) k_plain(PlainParams pp, const uint4* __
 
 // ---- resolves ----------------------------------------------------------------
 
+// The frame's list counters, reset for the next frame's cull by the resolve that
+// follows the last raster pass (a reset of its own in front of the cull cost
+// 1.8 us per frame; one by the raster's last CTA 4-40 % of the raster).  The two
+// item counts stay in `counts` for cr_last_frame_stats.
+__device__ __forceinline__ void finish_lists(uint32_t* scratch, uint32_t* counts) {
+    if (!scratch || blockIdx.x != 0 || threadIdx.x != 0) return;
+    counts[0] = scratch[kItemCount];
+    counts[1] = scratch[kItemCount2];
+    for (int k = 0; k < kCounterWords; k++) scratch[k] = 0u;
+}
+
 __device__ __forceinline__ bool depth_valid(uint64_t v) {
     float d = __uint_as_float((uint32_t)(v >> 32));
     return d > 0.0f && d < 1000000.0f;
@@ -658,7 +725,10 @@ __device__ __forceinline__ bool in_tiles(int64_t p, int32_t W, int32_t H) {
 __global__ void k_resolve_index(int64_t P, int64_t tail, uint64_t* __restrict__ fb,
                                 const uint32_t* __restrict__ rgba, int64_t rgba_words,
                                 uint32_t* __restrict__ image, int clear_after, uint64_t clear,
-                                int32_t W, int32_t H, int tiles) {
+                                int32_t W, int32_t H, int tiles,
+                                uint32_t* scratch, uint32_t* counts) {
+    grid_wait();
+    finish_lists(scratch, counts);
     int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int64_t p = 2 * t;
     if (p < P) {
@@ -691,7 +761,10 @@ __global__ void k_resolve_index(int64_t P, int64_t tail, uint64_t* __restrict__ 
 }
 
 __global__ void k_resolve_color(int64_t P, int64_t tail, uint64_t* __restrict__ fb,
-                                uint32_t* __restrict__ image, int clear_after, uint64_t clear) {
+                                uint32_t* __restrict__ image, int clear_after, uint64_t clear,
+                                uint32_t* scratch, uint32_t* counts) {
+    grid_wait();
+    finish_lists(scratch, counts);
     int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int64_t p = 2 * t;
     if (p < P) {
@@ -729,6 +802,7 @@ __device__ __forceinline__ uint32_t plain_rgba8(uint64_t v, int zero_rule) {
 __global__ void k_resolve_plain(int64_t P, int64_t tail, int32_t W, int32_t H, int tiles,
                                 int zero_rule, uint64_t* __restrict__ fb,
                                 uint32_t* __restrict__ image, int clear_after, uint64_t clear) {
+    grid_wait();
     int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t < P) {
         bool covered = true;
@@ -747,7 +821,10 @@ __global__ void k_resolve_plain(int64_t P, int64_t tail, int32_t W, int32_t H, i
 // compute_loop_las_hqs/resolve.cs:62-130
 __global__ void k_resolve_hqs(int64_t P, int64_t tail, uint32_t* __restrict__ depth,
                               uint64_t* __restrict__ accum, uint32_t* __restrict__ image,
-                              int clear_after) {
+                              int clear_after,
+                              uint32_t* scratch, uint32_t* counts) {
+    grid_wait();
+    finish_lists(scratch, counts);
     int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t < P) {
         ulonglong2 a = reinterpret_cast<const ulonglong2*>(accum)[t];
@@ -821,31 +898,50 @@ inline int blocks_for(int64_t n, int per) { return (int)((n + per - 1) / per); }
 
 }  // namespace
 
-int launch_file_records(const double view[16], const double proj[16], const double* box_min,
-                        int32_t nfiles, FileRec* out, void* stream, int float_uniforms, int literal) {
-    // the chunk travels by value in the kernel parameters: no staging buffer
-    // whose lifetime would have to outlast the launch
-    FileChunk c;
+template <int N>
+static int launch_file_chunk(const double view[16], const double pv[16], const double* box_min,
+                             int32_t first, int32_t count, FileRec* out, void* stream,
+                             int float_uniforms, int literal) {
+    FileChunk<N> c;
     c.float_uniforms = float_uniforms;
     c.literal = literal;
     for (int i = 0; i < 16; i++) {
+        c.pv[i] = pv[i];
         c.view[i] = view[i];
-        c.proj[i] = proj[i];
     }
-    for (int32_t first = 0; first < nfiles; first += kFilesPerLaunch) {
-        c.first = first;
-        c.count = std::min<int32_t>(kFilesPerLaunch, nfiles - first);
-        for (int k = 0; k < 3 * c.count; k++) c.box_min[k] = box_min[3 * (int64_t)first + k];
-        if (launch_k(k_file_records, blocks_for(c.count, 128), 128, (cudaStream_t)stream, c, out) != 0)
+    c.first = first;
+    c.count = count;
+    for (int k = 0; k < 3 * count; k++) c.box_min[k] = box_min[3 * (int64_t)first + k];
+    return launch_dep(k_file_records<N>, blocks_for(count, 8), 128, (cudaStream_t)stream, c, out);
+}
+
+int launch_file_records(const double view[16], const double proj[16], const double* box_min,
+                        int32_t nfiles, FileRec* out, void* stream, int float_uniforms, int literal) {
+    // proj * view as file_record and file_record_float form it
+    double pv[16];
+    if (float_uniforms) {
+        float fv[16], fp[16], fpv[16];
+        for (int i = 0; i < 16; i++) {
+            fv[i] = (float)view[i];
+            fp[i] = (float)proj[i];
+        }
+        mat_mul(fp, fv, fpv);
+        for (int i = 0; i < 16; i++) pv[i] = fpv[i];
+    } else {
+        mat_mul(proj, view, pv);
+    }
+    if (nfiles <= kFilesSmall) return launch_file_chunk<kFilesSmall>(view, pv, box_min, 0, nfiles, out, stream, float_uniforms, literal);
+    for (int32_t first = 0; first < nfiles; first += kFilesPerLaunch)
+        if (launch_file_chunk<kFilesPerLaunch>(view, pv, box_min, first, std::min<int32_t>(kFilesPerLaunch, nfiles - first),
+                                               out, stream, float_uniforms, literal) != 0)
             return -1;
-    }
     return 0;
 }
 
 int launch_cull(const ViewParams& vp, const cr_batch* batches, int64_t nb, int64_t capacity,
                 int32_t quirks, uint32_t* scratch, void* stream, int64_t list_cap, int node_slices) {
     if (nb <= 0) return 0;
-    return launch_k(k_cull, blocks_for(nb, 256), 256, (cudaStream_t)stream, vp, batches, nb,
+    return launch_dep(k_cull, blocks_for(nb, 256), 256, (cudaStream_t)stream, vp, batches, nb,
                     capacity, quirks, scratch, list_cap < 0 ? nb : list_cap, (int32_t)node_slices);
 }
 
@@ -873,20 +969,8 @@ static int launch_lists(const ViewParams& vp, const BatchedLaunch& bl, int grid,
     const int grid1 = std::min(grid, sms * occupancy_list1<MODE, PAYLOAD, BLOCK, MANY, LIT>());
     PairParams pp;
     fill_pair_params(vp, &pp);
-    if (launch_k(k_batched<MODE, PAYLOAD, BLOCK, 1, MANY, LIT>, grid1, BLOCK, s, vp, bl, pp) != 0) return -1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(BLOCK);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_batched<MODE, PAYLOAD, BLOCK, 0, MANY, LIT>, vp, bl, pp) == cudaSuccess
-               ? 0
-               : -1;
+    if (launch_dep(k_batched<MODE, PAYLOAD, BLOCK, 1, MANY, LIT>, grid1, BLOCK, s, vp, bl, pp) != 0) return -1;
+    return launch_dep(k_batched<MODE, PAYLOAD, BLOCK, 0, MANY, LIT>, grid, BLOCK, s, vp, bl, pp);
 }
 
 template <int MODE, int PAYLOAD>
@@ -958,46 +1042,46 @@ int launch_plain(const float T[16], int32_t W, int32_t H, const cr_vertex* v, in
     const uint4* v4 = reinterpret_cast<const uint4*>(v);
     cudaStream_t s = (cudaStream_t)stream;
     if (literal) {
-        if (variant == 1) return launch_k(k_plain<256, 1, true>, grid, 256, s, pp, v4, n, fb);
-        if (variant == 2) return launch_k(k_plain<256, 2, true>, grid, 256, s, pp, v4, n, fb);
-        return launch_k(k_plain<256, 0, true>, grid, 256, s, pp, v4, n, fb);
+        if (variant == 1) return launch_dep(k_plain<256, 1, true>, grid, 256, s, pp, v4, n, fb);
+        if (variant == 2) return launch_dep(k_plain<256, 2, true>, grid, 256, s, pp, v4, n, fb);
+        return launch_dep(k_plain<256, 0, true>, grid, 256, s, pp, v4, n, fb);
     }
-    if (variant == 1) return launch_k(k_plain<256, 1>, grid, 256, s, pp, v4, n, fb);
-    if (variant == 2) return launch_k(k_plain<256, 2>, grid, 256, s, pp, v4, n, fb);
-    return launch_k(k_plain<256, 0>, grid, 256, s, pp, v4, n, fb);
+    if (variant == 1) return launch_dep(k_plain<256, 1>, grid, 256, s, pp, v4, n, fb);
+    if (variant == 2) return launch_dep(k_plain<256, 2>, grid, 256, s, pp, v4, n, fb);
+    return launch_dep(k_plain<256, 0>, grid, 256, s, pp, v4, n, fb);
 }
 
 int launch_resolve_index(int32_t W, int32_t H, uint64_t* fb, const uint32_t* rgba,
                          int64_t rgba_words, uint32_t* image, int clear_after, uint64_t clear,
-                         void* stream, int tiles) {
+                         void* stream, int tiles, uint32_t* scratch, uint32_t* counts) {
     int64_t P = (int64_t)W * H, tail = (int64_t)W + 1;
     int64_t threads = (P + 1) / 2 > tail ? (P + 1) / 2 : tail;
-    return launch_k(k_resolve_index, blocks_for(threads, 256), 256, (cudaStream_t)stream, P, tail,
-                    fb, rgba, rgba_words, image, clear_after, clear, W, H, tiles);
+    return launch_dep(k_resolve_index, blocks_for(threads, 256), 256, (cudaStream_t)stream, P, tail,
+                    fb, rgba, rgba_words, image, clear_after, clear, W, H, tiles, scratch, counts);
 }
 
 int launch_resolve_color(int32_t W, int32_t H, uint64_t* fb, uint32_t* image, int clear_after,
-                         uint64_t clear, void* stream) {
+                         uint64_t clear, void* stream, uint32_t* scratch, uint32_t* counts) {
     int64_t P = (int64_t)W * H, tail = (int64_t)W + 1;
     int64_t threads = (P + 1) / 2 > tail ? (P + 1) / 2 : tail;
-    return launch_k(k_resolve_color, blocks_for(threads, 256), 256, (cudaStream_t)stream, P, tail,
-                    fb, image, clear_after, clear);
+    return launch_dep(k_resolve_color, blocks_for(threads, 256), 256, (cudaStream_t)stream, P, tail,
+                    fb, image, clear_after, clear, scratch, counts);
 }
 
 int launch_resolve_plain(int32_t W, int32_t H, uint64_t* fb, uint32_t* image, int clear_after,
                          uint64_t clear, int tiles, int zero_rule, void* stream) {
     int64_t P = (int64_t)W * H, tail = (int64_t)W + 1;
     int64_t threads = P > tail ? P : tail;
-    return launch_k(k_resolve_plain, blocks_for(threads, 256), 256, (cudaStream_t)stream, P, tail,
+    return launch_dep(k_resolve_plain, blocks_for(threads, 256), 256, (cudaStream_t)stream, P, tail,
                     W, H, tiles, zero_rule, fb, image, clear_after, clear);
 }
 
 int launch_resolve_hqs(int32_t W, int32_t H, uint32_t* depth, uint64_t* accum, uint32_t* image,
-                       int clear_after, void* stream) {
+                       int clear_after, void* stream, uint32_t* scratch, uint32_t* counts) {
     int64_t P = (int64_t)W * H, tail = (int64_t)W + 1;
     int64_t threads = P > tail ? P : tail;
-    return launch_k(k_resolve_hqs, blocks_for(threads, 256), 256, (cudaStream_t)stream, P, tail,
-                    depth, accum, image, clear_after);
+    return launch_dep(k_resolve_hqs, blocks_for(threads, 256), 256, (cudaStream_t)stream, P, tail,
+                    depth, accum, image, clear_after, scratch, counts);
 }
 
 int launch_check_reciprocal(uint64_t* bad, uint32_t* first) {

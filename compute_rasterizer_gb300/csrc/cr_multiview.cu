@@ -91,6 +91,7 @@ __global__ void __launch_bounds__(256) k_mv_cull(const MVView* __restrict__ view
                                                  int64_t capacity, int32_t quirks, int32_t culling,
                                                  int32_t lod_skip_level,
                                                  uint32_t* __restrict__ scratch) {
+    grid_wait();
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     bool keep = false;
     uint4 item = make_uint4(0, 0, 0, 0);
@@ -389,7 +390,7 @@ __device__ __forceinline__ void mv_raster_items(const MVArgs& a) {
         const Unit u = unit_range(ws, unit);
         const uint32_t wi = u.item;
         const int vb = u.vb, ve = u.ve;
-        const uint4 it = items[LIST == 0 ? (int64_t)wi : a.list_cap - 1 - (int64_t)wi];
+        const uint4 it = __ldcg(items + (LIST == 0 ? (int64_t)wi : a.list_cap - 1 - (int64_t)wi));
         const uint32_t b = it.x, g = it.y, vismask = it.z, levels = it.w;
         const int4* r4 = reinterpret_cast<const int4*>(a.batches + b);
         const int4 ra = __ldg(r4), rc = __ldg(r4 + 1), rd = __ldg(r4 + 2);
@@ -516,14 +517,18 @@ __device__ __forceinline__ void mv_raster_items(const MVArgs& a) {
     }
 }
 
-// List 1 is launched first and lets the list-0 grid start at once
-// (programmatic dependent launch); every list-0 CTA waits for the list-1 grid
-// before it exits, so the resolve that follows sees both lists' writes.
+// The grids are programmatic dependents of one another.  List 1 waits for the
+// cull, then lets the list-0 grid start at once; every list-0 CTA waits for the
+// list-1 grid before it exits, so the resolve that follows sees both lists'
+// writes.
 template <int PAYLOAD, int BLOCK, int LIST>
 __global__ void __launch_bounds__(BLOCK, (LIST == 0 ? 8 : 5) * 128 / BLOCK) k_mv_raster(MVArgs a) {
-    if (LIST == 1) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (LIST == 1) {
+        grid_wait();
+        grid_release();
+    }
     mv_raster_items<PAYLOAD, BLOCK, LIST>(a);
-    if (LIST == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (LIST == 0) grid_wait();
 }
 
 // Bound by its bytes (20 per pixel): 82M pixels of 64 views take 252 us, 6.5 TB/s.
@@ -537,6 +542,7 @@ __global__ void __launch_bounds__(256) k_mv_resolve(const MVView* __restrict__ v
                                                     const uint32_t* __restrict__ rgba,
                                                     int64_t rgba_words, int32_t payload,
                                                     int32_t clear_after, unsigned long long clear) {
+    grid_wait();
     const int32_t W = views[blockIdx.y].W, H = views[blockIdx.y].H;
     unsigned long long* fb = fbs + views[blockIdx.y].fb_off;
     uint32_t* image = images + views[blockIdx.y].img_off;
@@ -613,18 +619,10 @@ cudaError_t launch_mv_lists(const MVArgs& a, int grid, cudaStream_t s) {
     cudaGetDevice(&device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     const int grid1 = std::min(grid, sms * mv_occupancy_list1<PAYLOAD, BLOCK>());
-    if (launch_k(k_mv_raster<PAYLOAD, BLOCK, 1>, grid1, BLOCK, s, a) != 0) return cudaErrorLaunchFailure;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(BLOCK);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_mv_raster<PAYLOAD, BLOCK, 0>, a);
+    if (launch_dep(k_mv_raster<PAYLOAD, BLOCK, 1>, grid1, BLOCK, s, a) != 0 ||
+        launch_dep(k_mv_raster<PAYLOAD, BLOCK, 0>, grid, BLOCK, s, a) != 0)
+        return cudaErrorLaunchFailure;
+    return cudaSuccess;
 }
 
 template <int PAYLOAD>
@@ -698,7 +696,7 @@ cr_status mv_enqueue(const MVFrame& f, void* stream, const char** what) {
             return fail("file record launch");
     }
     if (threads > 0) {
-        if (launch_k(k_mv_cull, (unsigned)((threads + 255) / 256), 256, st, f.d_views, f.d_files,
+        if (launch_dep(k_mv_cull, (unsigned)((threads + 255) / 256), 256, st, f.d_views, f.d_files,
                      f.nviews, f.ci.nfiles, G, ngroups, f.ci.batches, nb, f.ci.capacity, f.quirks,
                      f.culling, f.lod_skip_level, f.scratch) != 0)
             return fail("cull launch");
@@ -732,7 +730,7 @@ cr_status mv_enqueue(const MVFrame& f, void* stream, const char** what) {
         const int64_t tiles = (words + 256 * kResolvePix - 1) / (256 * kResolvePix);
         const int64_t share = std::max<int64_t>((int64_t)f.num_sms * 64 / f.nviews, 1);
         const unsigned gx = (unsigned)std::min(tiles, share);
-        if (launch_k(k_mv_resolve, dim3(gx, (unsigned)f.nviews), 256, st, f.d_views,
+        if (launch_dep(k_mv_resolve, dim3(gx, (unsigned)f.nviews), 256, st, f.d_views,
                      reinterpret_cast<unsigned long long*>(f.fbs), f.images, f.ci.rgba, f.ci.capacity,
                      f.payload, f.clear_after, f.clear_value) != 0)
             return fail("resolve launch");
