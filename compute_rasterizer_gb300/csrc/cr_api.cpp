@@ -38,6 +38,7 @@ struct cr_ctx {
     // leaves them so; one without a resolve, or that failed on the way, does not
     bool counters_zero = false;
     bool captured = false;  // a frame was captured into a graph
+    cudaMemPool_t pool = nullptr;  // ctx_pool
     std::vector<cr_frame_events> timing;  // GLTimerQueries-style event pairs
     int32_t timing_used = 0;
     std::string last_error;
@@ -254,6 +255,22 @@ int cr::default_quirks_for(int32_t method) { return default_quirks(method); }
 
 int cr::ctx_device(const cr_ctx* ctx) { return ctx ? ctx->device : 0; }
 
+cudaMemPool_t cr::ctx_pool(cr_ctx* ctx) {
+    if (ctx->pool) return ctx->pool;
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = ctx->device;
+    cudaMemPool_t pool = nullptr;
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) return nullptr;
+    uint64_t keep = kPoolKeepBytes;
+    if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+        cudaMemPoolDestroy(pool);
+        return nullptr;
+    }
+    return ctx->pool = pool;
+}
+
 cr_status cr::view_params_for(const cr_view* view, const double* box_min, int32_t num_files,
                               int32_t culling, ViewParams* vp, int literal) {
     if (!view || !box_min || !vp || num_files < 1 || num_files > kMaxFiles)
@@ -388,6 +405,7 @@ cr_status cr_ctx_destroy(cr_ctx* ctx) {
     destroy_timing(ctx);
     if (ctx->scratch) cudaFree(ctx->scratch);
     if (ctx->files) cudaFree(ctx->files);
+    if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
     delete ctx;
     return CR_OK;
 }

@@ -212,6 +212,11 @@ cr_status encode_records_device(const uint8_t* d_rec, int64_t n, int32_t bpp, in
                                 uint32_t* d_lo, uint32_t* d_md, uint32_t* d_hi, uint32_t* d_rgba,
                                 void* stream);
 int ctx_device(const cr_ctx* ctx);
+// The context's pool of device memory for builders' temporary buffers, created on
+// first use; null if that fails.  Between uses it keeps up to kPoolKeepBytes, and
+// nothing once the context is destroyed.
+constexpr uint64_t kPoolKeepBytes = 4ull << 30;
+cudaMemPool_t ctx_pool(cr_ctx* ctx);
 
 // ---- multi-view frames (cr_multiview.cu), shared by cr_mv plans and the server
 

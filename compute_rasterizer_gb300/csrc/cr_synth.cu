@@ -203,12 +203,25 @@ __host__ __device__ inline uint64_t spread3(uint32_t a) {
     return x;
 }
 
+// The same for 10 and 11 bits.
+__host__ __device__ inline uint32_t spread10(uint32_t x) {
+    x = (x | x << 16) & 0x030000FFu;
+    x = (x | x << 8) & 0x0300F00Fu;
+    x = (x | x << 4) & 0x030C30C3u;
+    return (x | x << 2) & 0x09249249u;
+}
+__host__ __device__ inline uint32_t spread11(uint32_t x) { return spread10(x & 1023u) | (x >> 10) << 30; }
+
 struct MortonFrame {
     double min[3];
     double cube, inv;  // inv = RN(1 / cube)
     double scale[3];
     double offset[3];
-    cr::QuantFx fx[3];  // the GPU keys' integer form of morton_axis (cr_quant.h)
+    // the GPU keys' integer form of morton_axis (cr_quant.h): decides all but about
+    // one point in 10^5 per axis for LAS scales and extents; the host sort keeps the
+    // double chain, so every GPU/host comparison checks it
+    cr::QuantFx fx[3];
+    cr::QuantQuick qq[3];
 };
 
 // Sort_Frugal/src/main.cpp:82-105: normalise by the largest header extent.
@@ -235,19 +248,6 @@ __host__ __device__ inline uint64_t morton_of(const MortonFrame& f, const uint8_
     return spread3(q[0]) | (spread3(q[1]) << 1) | (spread3(q[2]) << 2);
 }
 
-// The GPU keys: the cell in integer arithmetic where the error bound decides
-// it (all but about one point in 10^5 per axis for LAS scales and extents),
-// else the double chain.  The host sort keeps the chain, so every GPU/host
-// comparison checks the integer form.
-__device__ inline uint64_t morton_of_fast(const MortonFrame& f, const uint8_t* rec) {
-    uint32_t q[3];
-    for (int k = 0; k < 3; k++) {
-        const int32_t X = get_i32(rec + 4 * k);
-        if (!cr::quant_fast(f.fx[k], X, 2097151u, &q[k])) q[k] = morton_axis(f, k, X);
-    }
-    return spread3(q[0]) | (spread3(q[1]) << 1) | (spread3(q[2]) << 2);
-}
-
 MortonFrame morton_frame(const cr_las_header* h) {
     MortonFrame f;
     double size[3];
@@ -260,8 +260,10 @@ MortonFrame morton_frame(const cr_las_header* h) {
     f.cube = std::max(std::max(size[0], size[1]), size[2]);
     if (!(f.cube > 0.0)) f.cube = 1.0;
     f.inv = 1.0 / f.cube;
-    for (int k = 0; k < 3; k++)
+    for (int k = 0; k < 3; k++) {
         f.fx[k] = cr::quant_setup(f.scale[k], f.offset[k], f.min[k], 0.0, false, f.cube, 21, INT32_MIN, INT32_MAX);
+        f.qq[k] = cr::quant_quick_setup(f.fx[k]);
+    }
     return f;
 }
 
@@ -316,12 +318,133 @@ __global__ void k_bounds(const uint8_t* rec, int64_t n, int32_t bpp, int32_t* mn
         }
 }
 
-__global__ void k_morton_keys(MortonFrame f, const uint8_t* rec, int64_t n, int32_t bpp,
-                              unsigned long long* keys, uint32_t* idx) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+// ---- record tiles in shared memory ----------------------------------------------
+//
+// LAS records are packed (26 bytes in format 2), so a thread that reads its own
+// record issues a load per byte or half word and a warp's loads share sectors:
+// the encoder and the keys were bound by those loads.  Here a CTA copies whole
+// tiles of records with 16-byte cp.async, one tile ahead of the one it works on,
+// and takes the fields from shared memory.
+
+constexpr int kTileBytes = 53248;  // the keys': two tiles per CTA, two CTAs per SM
+
+// Records per tile of `bytes`: whole 16-byte vectors, so every tile starts on one.
+inline int tile_records(int32_t bpp, int bytes) { return std::min(2048, bytes / bpp) & ~15; }
+
+// The int32 / uint16 at byte p of a tile; EVEN: every field starts on a half word.
+template <bool EVEN>
+__device__ __forceinline__ int32_t tile_i32(const uint8_t* p) {
+    if (!EVEN) return get_i32(p);
+    const uint16_t* h = reinterpret_cast<const uint16_t*>(p);
+    return (int32_t)((uint32_t)h[0] | ((uint32_t)h[1] << 16));
+}
+template <bool EVEN>
+__device__ __forceinline__ uint32_t tile_u16(const uint8_t* p) {
+    return EVEN ? *reinterpret_cast<const uint16_t*>(p) : get_u16(p);
+}
+
+// Starts the copy of `bytes` from the 16-byte aligned `src` to `dst` by the CTA.
+__device__ __forceinline__ void copy_tile(uint8_t* dst, const uint8_t* src, int bytes) {
+    const int vecs = bytes >> 4;
+    for (int k = threadIdx.x; k < vecs; k += blockDim.x) {
+        const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst + 16 * k);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src + 16 * (int64_t)k) : "memory");
+    }
+    for (int k = (vecs << 4) + threadIdx.x; k < bytes; k += blockDim.x) dst[k] = src[k];
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+// Waits for all but the newest `PENDING` copies.
+template <int PENDING>
+__device__ __forceinline__ void wait_tile() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
+    __syncthreads();
+}
+
+// A tile kernel's dynamic shared memory, allowed once per kernel and process.
+template <typename K>
+bool allow_shared(K kernel, int bytes) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
+}
+
+// Morton keys and identity permutation of records [0, n), and a copy of the
+// records for the gather to read: tiles go out again from shared memory, which
+// saves the copy of the sorted records back a read of its own.
+// (bpp even; copy null: none)
+__global__ void __launch_bounds__(512, 2) k_morton_keys(MortonFrame f, const uint8_t* __restrict__ rec, int64_t n,
+                                                        int32_t bpp, int tile_recs, unsigned long long* keys,
+                                                        uint32_t* idx, uint8_t* __restrict__ copy) {
+    extern __shared__ __align__(16) uint8_t s_tiles[];
+    const int64_t ntiles = (n + tile_recs - 1) / tile_recs;
+    auto recs = [&](int64_t t) { return (int)min((int64_t)tile_recs, n - t * tile_recs); };
+    int64_t t = blockIdx.x;
+    if (t < ntiles) copy_tile(s_tiles, rec + t * tile_recs * bpp, recs(t) * bpp);
+    for (int buf = 0; t < ntiles; t += gridDim.x, buf ^= 1) {
+        const int64_t next = t + gridDim.x;
+        if (next < ntiles) {
+            copy_tile(s_tiles + (buf ^ 1) * kTileBytes, rec + next * tile_recs * bpp, recs(next) * bpp);
+            wait_tile<1>();
+        } else {
+            wait_tile<0>();
+        }
+        const uint8_t* tile = s_tiles + buf * kTileBytes;
+        const int cnt = recs(t);
+        for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
+            uint32_t q[3];
+            for (int k = 0; k < 3; k++) {
+                const int32_t X = tile_i32<true>(tile + i * bpp + 4 * k);
+                if (!cr::quant_quick(f.qq[k], X, 2097151u, &q[k]) &&
+                    !cr::quant_fast(f.fx[k], X, 2097151u, &q[k]))
+                    q[k] = morton_axis(f, k, X);
+            }
+            // spread3 of the low 10 and the high 11 bits of each axis, in 32 bits
+            const uint32_t lo = spread10(q[0] & 1023u) | spread10(q[1] & 1023u) << 1 | spread10(q[2] & 1023u) << 2;
+            const uint32_t hx = spread11(q[0] >> 10), hy = spread11(q[1] >> 10), hz = spread11(q[2] >> 10);
+            const uint64_t hi = (uint64_t)hx | (uint64_t)hy << 1 | (uint64_t)hz << 2;
+            keys[t * tile_recs + i] = hi << 30 | lo;
+            idx[t * tile_recs + i] = (uint32_t)(t * tile_recs + i);
+        }
+        if (copy) {
+            uint8_t* out = copy + t * tile_recs * bpp;
+            const int bytes = cnt * bpp, vecs = bytes >> 4;
+            for (int k = threadIdx.x; k < vecs; k += blockDim.x)
+                reinterpret_cast<uint4*>(out)[k] = reinterpret_cast<const uint4*>(tile)[k];
+            for (int k = (vecs << 4) + threadIdx.x; k < bytes; k += blockDim.x) out[k] = tile[k];
+        }
+        __syncthreads();  // the tile is free for the copy after next
+    }
+}
+
+// Finishes a radix sort that left out the keys' lowest `low` bits: each run of
+// equal upper bits, in index order so far, is insertion-sorted by the whole key
+// (stable, so ties keep the index order).  Runs longer than kMaxRun raise *flag
+// and stay.  One thread per run; a run's neighbours compare upper bits only, which
+// no swap inside a run changes.
+constexpr int kMaxRun = 64;
+__global__ void __launch_bounds__(256) k_sort_runs(unsigned long long* keys, uint32_t* idx, int64_t n, int low,
+                                                   uint32_t* flag) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n - 1;
          i += (int64_t)gridDim.x * blockDim.x) {
-        keys[i] = morton_of_fast(f, rec + i * bpp);
-        idx[i] = (uint32_t)i;
+        const unsigned long long head = keys[i] >> low;
+        if (keys[i + 1] >> low != head || (i > 0 && keys[i - 1] >> low == head)) continue;
+        int len = 2;
+        while (i + len < n && len <= kMaxRun && keys[i + len] >> low == head) len++;
+        if (len > kMaxRun) {
+            *flag = 1u;
+            continue;
+        }
+        for (int k = 1; k < len; k++) {
+            const unsigned long long key = keys[i + k];
+            const uint32_t id = idx[i + k];
+            int j = k;
+            for (; j > 0 && keys[i + j - 1] > key; j--) {
+                keys[i + j] = keys[i + j - 1];
+                idx[i + j] = idx[i + j - 1];
+            }
+            if (j != k) {
+                keys[i + j] = key;
+                idx[i + j] = id;
+            }
+        }
     }
 }
 
@@ -331,13 +454,13 @@ __global__ void k_morton_keys(MortonFrame f, const uint8_t* rec, int64_t n, int3
 // slice of shared memory at their destination offsets, and the warp stores the
 // 32 * bpp contiguous destination bytes as 16-byte vectors (bpp is even, so
 // 32 * bpp is a multiple of 16 and the warp's first byte is 16-byte aligned
-// when dst is).  The tail warp (fewer than 32 records) stores 16-bit words.
+// when dst is: `vec`).  The tail warp (fewer than 32 records) stores 16-bit words.
 constexpr int kGatherMaxBpp = 64;
 constexpr int kGatherWarps = 8;
 __global__ void __launch_bounds__(32 * kGatherWarps) k_gather(const uint8_t* __restrict__ src,
                                                               uint8_t* __restrict__ dst,
                                                               const uint32_t* __restrict__ perm,
-                                                              int64_t n, int32_t bpp) {
+                                                              int64_t n, int32_t bpp, bool vec) {
     __shared__ __align__(16) uint16_t s_buf[kGatherWarps][32 * kGatherMaxBpp / 2];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint16_t* buf = s_buf[warp];
@@ -352,7 +475,7 @@ __global__ void __launch_bounds__(32 * kGatherWarps) k_gather(const uint8_t* __r
         }
         __syncwarp();
         uint8_t* d = dst + w0 * bpp;
-        if (cnt == 32) {
+        if (cnt == 32 && vec) {
             const int vecs = (32 * bpp) >> 4;
             for (int k = lane; k < vecs; k += 32)
                 reinterpret_cast<uint4*>(d)[k] = reinterpret_cast<const uint4*>(buf)[k];
@@ -385,28 +508,20 @@ __device__ __forceinline__ uint32_t quantize30(double d, double size, double inv
     return u < 1073741823u ? u : 1073741823u;
 }
 
-// LasLoaderSparse.cpp:84-199, one CTA per batch.
-__global__ void __launch_bounds__(256) k_encode(EncodeArgs a, const uint8_t* __restrict__ rec,
-                                                cr_batch* batches, uint32_t* lo, uint32_t* md,
-                                                uint32_t* hi, uint32_t* rgba) {
-    __shared__ int32_t s_red[6][8];
-    __shared__ double s_box[9];
-    __shared__ cr::QuantFx s_fx[3];
-    const int64_t first = (int64_t)blockIdx.x * cr::kPointsPerBatch;
-    const int64_t left = a.n - first;
-    const int cnt = (int)(left < cr::kPointsPerBatch ? left : cr::kPointsPerBatch);
-    // The batch AABB of v = double(X) * scale + offset - boxMin
-    // (LasLoaderSparse.cpp:93-105): every step rounds monotonically, so v is
-    // monotone in the integer X and the box is v at the integer extremes.
-    int32_t mn[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, mx[3] = {INT32_MIN, INT32_MIN, INT32_MIN};
-    for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
-        const uint8_t* r = rec + (first + i) * a.bpp;
-        for (int k = 0; k < 3; k++) {
-            const int32_t X = get_i32(r + 4 * k);
-            mn[k] = min(mn[k], X);
-            mx[k] = max(mx[k], X);
-        }
-    }
+// One batch's box and quantisation from the integer extremes, in shared memory.
+struct EncodeBox {
+    double box[9];  // min, max, 1 / size
+    cr::QuantFx fx[3];
+    cr::QuantQuick qq[3];
+};
+
+// Writes a batch's record and the shared box from each thread's extremes.
+// The batch AABB of v = double(X) * scale + offset - boxMin
+// (LasLoaderSparse.cpp:93-105): every step rounds monotonically, so v is
+// monotone in the integer X and the box is v at the integer extremes.
+__device__ __forceinline__ void encode_box(const EncodeArgs& a, int32_t mn[3], int32_t mx[3], int64_t first,
+                                           int cnt, cr_batch* batches, EncodeBox& s_b) {
+    __shared__ int32_t s_red[6][32];
     for (int o = 16; o > 0; o >>= 1)
         for (int k = 0; k < 3; k++) {
             mn[k] = min(mn[k], __shfl_xor_sync(0xFFFFFFFFu, mn[k], o));
@@ -429,51 +544,165 @@ __global__ void __launch_bounds__(256) k_encode(EncodeArgs a, const uint8_t* __r
         const double vlo = (double)lo * a.scale[k] + a.offset[k] - a.box_min[k];
         const double vhi = (double)hi * a.scale[k] + a.offset[k] - a.box_min[k];
         const double b0 = a.scale[k] < 0.0 ? vhi : vlo, b1 = a.scale[k] < 0.0 ? vlo : vhi;
-        s_box[k] = b0;
-        s_box[3 + k] = b1;
-        s_box[6 + k] = 1.0 / (b1 - b0);
-        s_fx[k] = cr::quant_setup(a.scale[k], a.offset[k], a.box_min[k], b0, true, b1 - b0, 30, lo, hi);
+        s_b.box[k] = b0;
+        s_b.box[3 + k] = b1;
+        s_b.box[6 + k] = 1.0 / (b1 - b0);
+        s_b.fx[k] = cr::quant_setup(a.scale[k], a.offset[k], a.box_min[k], b0, true, b1 - b0, 30, lo, hi);
+        s_b.qq[k] = cr::quant_quick_setup(s_b.fx[k]);
     }
     __syncthreads();
-    const double bmin[3] = {s_box[0], s_box[1], s_box[2]};
-    const double size[3] = {s_box[3] - s_box[0], s_box[4] - s_box[1], s_box[5] - s_box[2]};
-    const double inv[3] = {s_box[6], s_box[7], s_box[8]};
     if (threadIdx.x == 0) {
         cr_batch b;
         memset(&b, 0, sizeof(b));
-        b.min_x = (float)s_box[0]; b.min_y = (float)s_box[1]; b.min_z = (float)s_box[2];
-        b.max_x = (float)s_box[3]; b.max_y = (float)s_box[4]; b.max_z = (float)s_box[5];
+        b.min_x = (float)s_b.box[0]; b.min_y = (float)s_b.box[1]; b.min_z = (float)s_b.box[2];
+        b.max_x = (float)s_b.box[3]; b.max_y = (float)s_b.box[4]; b.max_z = (float)s_b.box[5];
         b.num_points = cnt;
         b.first_point = (int32_t)(a.sparse_offset + first);
         b.file_index = a.file_index;
         batches[blockIdx.x] = b;
     }
-    // Each coordinate's 30-bit cell in integer arithmetic where the error bound
-    // decides it (cr_quant.h), else the double chain: the same integer either way.
-    for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
-        const int64_t pi = first + i;
-        const uint8_t* r = rec + pi * a.bpp;
-        uint32_t q[3];
-        for (int k = 0; k < 3; k++) {
-            const int32_t X = get_i32(r + 4 * k);
-            if (!cr::quant_fast(s_fx[k], X, 1073741823u, &q[k])) {
-                const double v = (double)X * a.scale[k] + a.offset[k] - a.box_min[k];
-                q[k] = quantize30(v - bmin[k], size[k], inv[k]);
-            }
-        }
-        lo[pi] = ((q[0] >> 20) & 1023u) | (((q[1] >> 20) & 1023u) << 10) | (((q[2] >> 20) & 1023u) << 20);
-        md[pi] = ((q[0] >> 10) & 1023u) | (((q[1] >> 10) & 1023u) << 10) | (((q[2] >> 10) & 1023u) << 20);
-        hi[pi] = (q[0] & 1023u) | ((q[1] & 1023u) << 10) | ((q[2] & 1023u) << 20);
-        if (a.rgb >= 0) {
-            uint32_t R = get_u16(r + a.rgb), G = get_u16(r + a.rgb + 2), B = get_u16(r + a.rgb + 4);
-            R = R < 256u ? R : R / 256u;
-            G = G < 256u ? G : G / 256u;
-            B = B < 256u ? B : B / 256u;
-            rgba[pi] = R | (G << 8) | (B << 16);
-        } else {
-            rgba[pi] = 0u;
-        }
+}
+
+// One point to word `pi` of the streams, from its integer coordinates X (a
+// callable of the axis) and its color word.  Each coordinate's 30-bit cell in
+// integer arithmetic where the error bound decides it (cr_quant.h), else the
+// double chain: the same integer either way.
+// The rest of the points, out of line: it would cost the common path registers.
+__device__ __noinline__ uint32_t encode_exact(const EncodeArgs& a, const EncodeBox& s_b, int k, int32_t x) {
+    uint32_t q;
+    if (cr::quant_fast(s_b.fx[k], x, 1073741823u, &q)) return q;
+    const double v = (double)x * a.scale[k] + a.offset[k] - a.box_min[k];
+    return quantize30(v - s_b.box[k], s_b.box[3 + k] - s_b.box[k], s_b.box[6 + k]);
+}
+
+template <typename F>
+__device__ __forceinline__ void encode_point(const EncodeArgs& a, const EncodeBox& s_b, F X, uint32_t color,
+                                             int64_t pi, uint32_t* lo, uint32_t* md, uint32_t* hi, uint32_t* rgba) {
+    uint32_t l = 0, m = 0, h = 0;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const int32_t x = X(k);
+        uint32_t q;
+        if (!cr::quant_quick(s_b.qq[k], x, 1073741823u, &q)) q = encode_exact(a, s_b, k, x);
+        l |= ((q >> 20) & 1023u) << (10 * k);
+        m |= ((q >> 10) & 1023u) << (10 * k);
+        h |= (q & 1023u) << (10 * k);
     }
+    lo[pi] = l;
+    md[pi] = m;
+    hi[pi] = h;
+    rgba[pi] = color;
+}
+
+// The color word of a record (LasLoaderSparse.cpp:133-144).
+template <bool EVEN>
+__device__ __forceinline__ uint32_t encode_color(const EncodeArgs& a, const uint8_t* r) {
+    if (a.rgb < 0) return 0u;
+    uint32_t R = tile_u16<EVEN>(r + a.rgb), G = tile_u16<EVEN>(r + a.rgb + 2), B = tile_u16<EVEN>(r + a.rgb + 4);
+    R = R < 256u ? R : R / 256u;
+    G = G < 256u ? G : G / 256u;
+    B = B < 256u ? B : B / 256u;
+    return R | (G << 8) | (B << 16);
+}
+
+// LasLoaderSparse.cpp:84-199, one CTA per batch: its extremes, then its points,
+// over a ring of STAGES tiles in shared memory.  The second walk runs backwards
+// from the tiles that are still there.
+//
+// Reading each field from global memory (12 byte loads per record and walk) and
+// quantising in 421 warp instructions per 32 points held it at 2.4 TB/s; tiles and
+// quant_quick (one third of the instructions) leave the barriers and the box's
+// serial double chain, which four small CTAs per SM cover: 40M records 1109 -> 523
+// us, 200M 5329 -> 2288 (3.7 TB/s).  With few batches nothing covers them, and
+// fewer, wider CTAs whose rings hold more of their batch are faster: at most one
+// per SM (a load task of the LAS loader is 100) 1.0M records 65.5 -> 61 and 300k
+// 52.8 -> 38, at most two 2M 108 -> 103 (EncodeMany 115).
+template <int THREADS, int CTAS, int STAGES, int TILE_BYTES>
+struct EncodeShape {
+    static constexpr int kThreads = THREADS, kCtas = CTAS, kStages = STAGES, kBytes = TILE_BYTES;
+    static constexpr int kShared = STAGES * TILE_BYTES;
+};
+using EncodeMany = EncodeShape<256, 4, 2, 26624>;
+using EncodeTwo = EncodeShape<512, 2, 2, 53248>;
+using EncodeFew = EncodeShape<1024, 1, 4, 53248>;
+
+template <bool EVEN, typename S>
+__global__ void __launch_bounds__(S::kThreads, S::kCtas) k_encode(EncodeArgs a, const uint8_t* __restrict__ rec,
+                                                                  int tile_recs, cr_batch* batches, uint32_t* lo,
+                                                                  uint32_t* md, uint32_t* hi, uint32_t* rgba) {
+    extern __shared__ __align__(16) uint8_t s_tiles[];
+    __shared__ EncodeBox s_b;
+    const int64_t first = (int64_t)blockIdx.x * cr::kPointsPerBatch;
+    const int cnt = (int)min((int64_t)cr::kPointsPerBatch, a.n - first);
+    const uint8_t* src = rec + first * a.bpp;
+    const int ntiles = (cnt + tile_recs - 1) / tile_recs;
+    auto recs = [&](int t) { return min(tile_recs, cnt - t * tile_recs); };
+    auto tile = [&](int t) { return s_tiles + (t % S::kStages) * S::kBytes; };
+    // one copy group per call, empty outside the batch, so the waits count alike
+    auto fetch = [&](int t) {
+        copy_tile(tile(max(t, 0)), src + (int64_t)t * tile_recs * a.bpp, t >= 0 && t < ntiles ? recs(t) * a.bpp : 0);
+    };
+    int32_t mn[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, mx[3] = {INT32_MIN, INT32_MIN, INT32_MIN};
+    for (int t = 0; t < S::kStages - 1; t++) fetch(t);
+    for (int t = 0; t < ntiles; t++) {
+        fetch(t + S::kStages - 1);
+        wait_tile<S::kStages - 1>();
+        const uint8_t* r = tile(t);
+        const int m = recs(t);
+        for (int i = threadIdx.x; i < m; i += S::kThreads)
+            for (int k = 0; k < 3; k++) {
+                const int32_t X = tile_i32<EVEN>(r + i * a.bpp + 4 * k);
+                mn[k] = min(mn[k], X);
+                mx[k] = max(mx[k], X);
+            }
+        __syncthreads();
+    }
+    encode_box(a, mn, mx, first, cnt, batches, s_b);
+    for (int t = ntiles - 1; t >= 0; t--) {
+        if (t < ntiles - S::kStages) wait_tile<S::kStages - 1>();
+        const int m = recs(t);
+        for (int i = threadIdx.x; i < m; i += S::kThreads) {
+            const uint8_t* r = tile(t) + i * a.bpp;
+            encode_point(a, s_b, [&](int k) { return tile_i32<EVEN>(r + 4 * k); }, encode_color<EVEN>(a, r),
+                         first + (int64_t)t * tile_recs + i, lo, md, hi, rgba);
+        }
+        __syncthreads();
+        fetch(t - S::kStages);
+    }
+}
+
+template <typename S>
+cudaError_t launch_encode(const EncodeArgs& a, const uint8_t* rec, cr_batch* batches, uint32_t* lo, uint32_t* md,
+                          uint32_t* hi, uint32_t* rgba, unsigned nb, cudaStream_t s) {
+    static const bool allowed = allow_shared(k_encode<true, S>, S::kShared) && allow_shared(k_encode<false, S>, S::kShared);
+    if (!allowed) return cudaErrorInvalidConfiguration;
+    const int tile = tile_records(a.bpp, S::kBytes);
+    if ((a.bpp & 1) == 0 && (a.rgb < 0 || (a.rgb & 1) == 0))
+        k_encode<true, S><<<nb, S::kThreads, S::kShared, s>>>(a, rec, tile, batches, lo, md, hi, rgba);
+    else
+        k_encode<false, S><<<nb, S::kThreads, S::kShared, s>>>(a, rec, tile, batches, lo, md, hi, rgba);
+    return cudaGetLastError();
+}
+
+// The same straight from global memory, a load per byte: records that do not start
+// on a 16-byte boundary, or too long for a tile.
+__global__ void __launch_bounds__(256) k_encode_bytes(EncodeArgs a, const uint8_t* __restrict__ rec,
+                                                      cr_batch* batches, uint32_t* lo, uint32_t* md, uint32_t* hi,
+                                                      uint32_t* rgba) {
+    __shared__ EncodeBox s_b;
+    const int64_t first = (int64_t)blockIdx.x * cr::kPointsPerBatch;
+    const int cnt = (int)min((int64_t)cr::kPointsPerBatch, a.n - first);
+    int32_t mn[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, mx[3] = {INT32_MIN, INT32_MIN, INT32_MIN};
+    for (int i = threadIdx.x; i < cnt; i += blockDim.x)
+        for (int k = 0; k < 3; k++) {
+            const int32_t X = get_i32(rec + (first + i) * a.bpp + 4 * k);
+            mn[k] = min(mn[k], X);
+            mx[k] = max(mx[k], X);
+        }
+    encode_box(a, mn, mx, first, cnt, batches, s_b);
+    for (int i = threadIdx.x; i < cnt; i += blockDim.x)
+        encode_point(a, s_b, [&](int k) { return get_i32(rec + (first + i) * a.bpp + 4 * k); },
+                     encode_color<false>(a, rec + (first + i) * a.bpp), first + i, lo, md, hi, rgba);
 }
 
 __host__ __device__ inline cr_vertex uniform_vertex(uint64_t seed, uint64_t i, float size) {
@@ -539,8 +768,21 @@ cr_status cr::encode_records_device(const uint8_t* d_rec, int64_t n, int32_t bpp
     a.bpp = bpp;
     a.rgb = rgb < 0 ? -1 : rgb;
     a.file_index = file_index;
-    k_encode<<<(unsigned)nb, 256, 0, (cudaStream_t)stream>>>(a, d_rec, d_batches, d_lo, d_md, d_hi, d_rgba);
-    return cuda_status(cudaGetLastError());
+    cudaStream_t s = (cudaStream_t)stream;
+    if (tile_records(bpp, EncodeMany::kBytes) == 0 || (reinterpret_cast<uintptr_t>(d_rec) & 15) != 0) {
+        k_encode_bytes<<<(unsigned)nb, 256, 0, s>>>(a, d_rec, d_batches, d_lo, d_md, d_hi, d_rgba);
+        return cuda_status(cudaGetLastError());
+    }
+    int device = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    if (e == cudaSuccess) {
+        const auto launch = nb <= sms       ? launch_encode<EncodeFew>
+                            : nb <= 2 * sms ? launch_encode<EncodeTwo>
+                                            : launch_encode<EncodeMany>;
+        e = launch(a, d_rec, d_batches, d_lo, d_md, d_hi, d_rgba, (unsigned)nb, s);
+    }
+    return cuda_status(e);
 }
 
 extern "C" {
@@ -632,38 +874,73 @@ cr_status cr_morton_sort_device(cr_ctx* ctx, uint8_t* d_rec, int64_t n, int32_t 
     if (n <= 1) return CR_OK;
     cudaStream_t s = (cudaStream_t)stream;
     const MortonFrame f = morton_frame(hdr);
-    unsigned long long *k0 = nullptr, *k1 = nullptr;
-    uint32_t *v0 = nullptr, *v1 = nullptr;
-    uint8_t* tmp = nullptr;
-    void* cub_tmp = nullptr;
+    // The sort's buffers in one allocation of the context's pool (six of their own
+    // took 2 ms of a 40M-point sort in the driver): keys and indices twice, the
+    // radix sort's own, a copy of the records (the gather reads it and writes d_rec
+    // in place), a flag.
+    const cudaMemPool_t pool = cr::ctx_pool(ctx);
+    if (!pool) return CR_ERR_CUDA;
+    cub::DoubleBuffer<unsigned long long> keys;
+    cub::DoubleBuffer<uint32_t> vals;
     size_t cub_bytes = 0;
-    cudaError_t e = cudaMalloc(&k0, n * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&k1, n * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&v0, n * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&v1, n * 4);
+    cudaError_t e = cub::DeviceRadixSort::SortPairs(nullptr, cub_bytes, keys, vals, (int)n, 0, 63, s);
+    if (e != cudaSuccess) return cuda_status(e);
+    const auto padded = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
+    const size_t key_bytes = padded((size_t)n * 8), val_bytes = padded((size_t)n * 4);
+    uint8_t* buf = nullptr;
+    e = cudaMallocFromPoolAsync(
+        reinterpret_cast<void**>(&buf),
+        2 * key_bytes + 2 * val_bytes + padded(cub_bytes) + padded((size_t)n * bpp) + 256, pool, s);
+    if (e != cudaSuccess) return cuda_status(e);
+    uint8_t* at = buf;
+    const auto take = [&at](size_t bytes) {
+        uint8_t* p = at;
+        at += bytes;
+        return p;
+    };
+    for (auto& k : keys.d_buffers) k = reinterpret_cast<unsigned long long*>(take(key_bytes));
+    for (auto& v : vals.d_buffers) v = reinterpret_cast<uint32_t*>(take(val_bytes));
+    void* cub_tmp = take(padded(cub_bytes));
+    uint32_t* flag = reinterpret_cast<uint32_t*>(take(256));
+    uint8_t* copy = at;
+    // tiles start on 16 bytes: records that do not are copied to where they do first
+    const bool aligned = (reinterpret_cast<uintptr_t>(d_rec) & 15) == 0;
+    if (!aligned) e = cudaMemcpyAsync(copy, d_rec, (size_t)n * bpp, cudaMemcpyDeviceToDevice, s);
+    static const bool tiles = allow_shared(k_morton_keys, 2 * kTileBytes);
+    if (e == cudaSuccess && !tiles) e = cudaErrorInvalidConfiguration;
     if (e == cudaSuccess) {
-        k_morton_keys<<<grid_for(n), 256, 0, s>>>(f, d_rec, n, bpp, k0, v0);
+        const int tile = tile_records(bpp, kTileBytes);  // bpp <= kGatherMaxBpp: at least 832
+        const int grid = (int)std::min<int64_t>((n + tile - 1) / tile, 2 * (int64_t)cr_ctx_num_sms(ctx));
+        k_morton_keys<<<grid, 512, 2 * kTileBytes, s>>>(f, aligned ? d_rec : copy, n, bpp, tile, keys.Current(),
+                                                        vals.Current(), aligned ? copy : nullptr);
         e = cudaGetLastError();
     }
-    cub::DoubleBuffer<unsigned long long> keys(k0, k1);
-    cub::DoubleBuffer<uint32_t> vals(v0, v1);
+    // Radix passes over the upper 40 bits (48 above 2^26 points), 5 (6) in place of 8
+    // at 0.3 ms each for 40M points; k_sort_runs (0.1 ms) finishes the runs they leave
+    // equal.  A surface scan fills about two bits of three, so 40 bits are 2^26
+    // cells and runs stay short; points so clustered that a run passes kMaxRun get
+    // the passes over all bits after all.
+    const int low = n <= ((int64_t)1 << 26) ? 23 : 15;
+    uint32_t long_runs = 0;
+    if (e == cudaSuccess) e = cudaMemsetAsync(flag, 0, 4, s);
     if (e == cudaSuccess)
-        e = cub::DeviceRadixSort::SortPairs(nullptr, cub_bytes, keys, vals, (int)n, 0, 63, s);
-    if (e == cudaSuccess) e = cudaMalloc(&cub_tmp, cub_bytes);
-    if (e == cudaSuccess)
+        e = cub::DeviceRadixSort::SortPairs(cub_tmp, cub_bytes, keys, vals, (int)n, low, 63, s);
+    if (e == cudaSuccess) {
+        k_sort_runs<<<grid_for(n), 256, 0, s>>>(keys.Current(), vals.Current(), n, low, flag);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&long_runs, flag, 4, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e == cudaSuccess && long_runs)
         e = cub::DeviceRadixSort::SortPairs(cub_tmp, cub_bytes, keys, vals, (int)n, 0, 63, s);
-    if (e == cudaSuccess) e = cudaMalloc(&tmp, (size_t)n * bpp);
     if (e == cudaSuccess) {
         const int64_t warps = (n + 31) / 32;
         const int grid = (int)std::min<int64_t>((warps + kGatherWarps - 1) / kGatherWarps, 65535);
-        k_gather<<<grid, 32 * kGatherWarps, 0, s>>>(d_rec, tmp, vals.Current(), n, bpp);
+        k_gather<<<grid, 32 * kGatherWarps, 0, s>>>(copy, d_rec, vals.Current(), n, bpp, aligned);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_rec, tmp, (size_t)n * bpp, cudaMemcpyDeviceToDevice, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    void* ptrs[6] = {k0, k1, v0, v1, tmp, cub_tmp};
-    for (void* q : ptrs)
-        if (q) cudaFree(q);
+    cudaFreeAsync(buf, s);
     return cuda_status(e);
 }
 
