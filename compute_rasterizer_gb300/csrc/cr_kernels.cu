@@ -713,75 +713,86 @@ __device__ __forceinline__ bool depth_valid(uint64_t v) {
 
 // Whether pixel p lies in the floor(W/16) x floor(H/16) tiles a resolve of
 // 16x16 groups covers (CR_QUIRK_RESOLVE_TILES).
-__device__ __forceinline__ bool in_tiles(int64_t p, int32_t W, int32_t H) {
-    const int64_t y = p / W, x = p - y * W;
-    return x < (W & ~15) && y < (H & ~15);
+__device__ __forceinline__ bool in_tiles(uint32_t p, int32_t W, int32_t H) {
+    const uint32_t y = p / (uint32_t)W, x = p - y * (uint32_t)W;
+    return x < (uint32_t)(W & ~15) && y < (uint32_t)(H & ~15);
 }
 
-// resolve.cs:100-146 (index payload) -- 2 pixels per thread.  tiles: only the
-// pixels of full 16x16 tiles are resolved (compute_loop_nodes.h:199-201); the
-// re-clear covers every pixel (loop_nodes clears separately,
-// compute_loop_nodes.h:239-251).
-__global__ void k_resolve_index(int64_t P, int64_t tail, uint64_t* __restrict__ fb,
-                                const uint32_t* __restrict__ rgba, int64_t rgba_words,
-                                uint32_t* __restrict__ image, int clear_after, uint64_t clear,
-                                int32_t W, int32_t H, int tiles,
-                                uint32_t* scratch, uint32_t* counts) {
-    grid_wait();
-    finish_lists(scratch, counts);
-    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    int64_t p = 2 * t;
-    if (p < P) {
-        if (tiles) {
-            for (int64_t q = p; q < p + 2 && q < P; q++) {
-                if (in_tiles(q, W, H)) {
-                    const uint64_t v = fb[q];
-                    const uint32_t i0 = depth_valid(v) ? (uint32_t)v : 0u;
-                    image[q] = (i0 == 0u || i0 >= rgba_words) ? kBackground : __ldg(rgba + i0);
-                }
-                if (clear_after) fb[q] = clear;
-            }
-        } else if (p + 1 < P) {
-            ulonglong2 v = reinterpret_cast<const ulonglong2*>(fb)[t];
-            uint32_t i0 = depth_valid(v.x) ? (uint32_t)v.x : 0u;
-            uint32_t i1 = depth_valid(v.y) ? (uint32_t)v.y : 0u;
-            uint2 o;
-            o.x = (i0 == 0u || i0 >= rgba_words) ? kBackground : __ldg(rgba + i0);
-            o.y = (i1 == 0u || i1 >= rgba_words) ? kBackground : __ldg(rgba + i1);
-            reinterpret_cast<uint2*>(image)[t] = o;
-            if (clear_after) reinterpret_cast<ulonglong2*>(fb)[t] = make_ulonglong2(clear, clear);
+// The u64 resolves: kPairs pairs of pixels per thread, a CTA apart, every load of a
+// thread in flight before its first is used.  A frame's words are still in L2 and
+// the grids are bound by latency: frames with 4 pairs against 1 (and the plain
+// methods' one pixel and 64-bit division per thread) octree of 2M 33.4 -> 30.6 us,
+// plain 4M 42.4 -> 39.2, 4K ground pose 85.8 -> 83.9.  `color(word, pixel)` is the image word; `covered(pixel)` false keeps the
+// pixel's image word (and, with KEEP, its framebuffer word).
+constexpr int kPairs = 4, kResolveBlock = 256;
+template <bool KEEP, typename Color, typename Covered>
+__device__ __forceinline__ void resolve_words(int64_t P, int64_t tail, uint64_t* __restrict__ fb,
+                                              uint32_t* __restrict__ image, int clear_after, uint64_t clear,
+                                              Color color, Covered covered) {
+    const uint32_t pairs = (uint32_t)((P + 1) / 2);  // P < 2^31
+    const uint32_t t0 = blockIdx.x * (kPairs * kResolveBlock) + threadIdx.x;
+    ulonglong2 v[kPairs];
+#pragma unroll
+    for (int k = 0; k < kPairs; k++) {
+        const uint32_t t = t0 + k * kResolveBlock;
+        // the word after an odd P's last pixel is the guard tail's first
+        if (t < pairs) v[k] = reinterpret_cast<const ulonglong2*>(fb)[t];
+    }
+#pragma unroll
+    for (int k = 0; k < kPairs; k++) {
+        const uint32_t t = t0 + k * kResolveBlock, p = 2 * t;
+        if (t >= pairs) break;
+        const bool two = p + 1 < P;
+        const bool c0 = covered(p), c1 = two && covered(p + 1);
+        if (c0 && c1) {
+            reinterpret_cast<uint2*>(image)[t] = make_uint2(color(v[k].x), color(v[k].y));
         } else {
-            uint64_t v = fb[p];
-            uint32_t i0 = depth_valid(v) ? (uint32_t)v : 0u;
-            image[p] = (i0 == 0u || i0 >= rgba_words) ? kBackground : __ldg(rgba + i0);
-            if (clear_after) fb[p] = clear;
+            if (c0) image[p] = color(v[k].x);
+            if (c1) image[p + 1] = color(v[k].y);
+        }
+        if (!clear_after) continue;
+        const bool k0 = !KEEP || c0, k1 = two && (!KEEP || c1);
+        if (k0 && k1) {
+            reinterpret_cast<ulonglong2*>(fb)[t] = make_ulonglong2(clear, clear);
+        } else {
+            if (k0) fb[p] = clear;
+            if (k1) fb[p + 1] = clear;
         }
     }
-    if (clear_after && t < tail) fb[P + t] = clear;
+    if (!clear_after || tail <= 0) return;
+    for (int64_t t = (int64_t)blockIdx.x * kResolveBlock + threadIdx.x; t < tail;
+         t += (int64_t)gridDim.x * kResolveBlock)
+        fb[P + t] = clear;
 }
 
-__global__ void k_resolve_color(int64_t P, int64_t tail, uint64_t* __restrict__ fb,
-                                uint32_t* __restrict__ image, int clear_after, uint64_t clear,
-                                uint32_t* scratch, uint32_t* counts) {
+// resolve.cs:100-146 (index payload).  tiles: only the pixels of full 16x16 tiles
+// are resolved (compute_loop_nodes.h:199-201); the re-clear covers every pixel
+// (loop_nodes clears separately, compute_loop_nodes.h:239-251).
+__global__ void __launch_bounds__(kResolveBlock)
+    k_resolve_index(int64_t P, int64_t tail, uint64_t* __restrict__ fb, const uint32_t* __restrict__ rgba,
+                    int64_t rgba_words, uint32_t* __restrict__ image, int clear_after, uint64_t clear, int32_t W,
+                    int32_t H, int tiles, uint32_t* scratch, uint32_t* counts) {
     grid_wait();
     finish_lists(scratch, counts);
-    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    int64_t p = 2 * t;
-    if (p < P) {
-        if (p + 1 < P) {
-            ulonglong2 v = reinterpret_cast<const ulonglong2*>(fb)[t];
-            uint2 o;
-            o.x = depth_valid(v.x) ? (uint32_t)v.x : kBackground;
-            o.y = depth_valid(v.y) ? (uint32_t)v.y : kBackground;
-            reinterpret_cast<uint2*>(image)[t] = o;
-            if (clear_after) reinterpret_cast<ulonglong2*>(fb)[t] = make_ulonglong2(clear, clear);
-        } else {
-            uint64_t v = fb[p];
-            image[p] = depth_valid(v) ? (uint32_t)v : kBackground;
-            if (clear_after) fb[p] = clear;
-        }
-    }
-    if (clear_after && t < tail) fb[P + t] = clear;
+    const auto color = [=](uint64_t v) {
+        const uint32_t i = depth_valid(v) ? (uint32_t)v : 0u;
+        return i == 0u || i >= rgba_words ? kBackground : __ldg(rgba + i);
+    };
+    if (tiles)
+        resolve_words<false>(P, tail, fb, image, clear_after, clear, color,
+                             [=](uint32_t p) { return in_tiles(p, W, H); });
+    else
+        resolve_words<false>(P, tail, fb, image, clear_after, clear, color, [](uint32_t) { return true; });
+}
+
+__global__ void __launch_bounds__(kResolveBlock)
+    k_resolve_color(int64_t P, int64_t tail, uint64_t* __restrict__ fb, uint32_t* __restrict__ image,
+                    int clear_after, uint64_t clear, uint32_t* scratch, uint32_t* counts) {
+    grid_wait();
+    finish_lists(scratch, counts);
+    resolve_words<false>(P, tail, fb, image, clear_after, clear,
+                         [](uint64_t v) { return depth_valid(v) ? (uint32_t)v : kBackground; },
+                         [](uint32_t) { return true; });
 }
 
 // compute_2021_earlyz/resolve.cs:41-77
@@ -799,23 +810,16 @@ __device__ __forceinline__ uint32_t plain_rgba8(uint64_t v, int zero_rule) {
 // floor(H/16) tiles of 16x16 that the reference dispatches
 // (compute_2021_earlyz.h:161-163) are resolved and re-cleared; every other
 // image and framebuffer word, the guard tail included, keeps its value.
-__global__ void k_resolve_plain(int64_t P, int64_t tail, int32_t W, int32_t H, int tiles,
-                                int zero_rule, uint64_t* __restrict__ fb,
-                                uint32_t* __restrict__ image, int clear_after, uint64_t clear) {
+__global__ void __launch_bounds__(kResolveBlock)
+    k_resolve_plain(int64_t P, int64_t tail, int32_t W, int32_t H, int tiles, int zero_rule,
+                    uint64_t* __restrict__ fb, uint32_t* __restrict__ image, int clear_after, uint64_t clear) {
     grid_wait();
-    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < P) {
-        bool covered = true;
-        if (tiles) {
-            const int64_t y = t / W, x = t - y * W;
-            covered = x < (W & ~15) && y < (H & ~15);
-        }
-        if (covered) {
-            image[t] = plain_rgba8(fb[t], zero_rule);
-            if (clear_after) fb[t] = clear;
-        }
-    }
-    if (clear_after && !tiles && t < tail) fb[P + t] = clear;
+    const auto color = [=](uint64_t v) { return plain_rgba8(v, zero_rule); };
+    if (tiles)
+        resolve_words<true>(P, 0, fb, image, clear_after, clear, color,
+                            [=](uint32_t p) { return in_tiles(p, W, H); });
+    else
+        resolve_words<true>(P, tail, fb, image, clear_after, clear, color, [](uint32_t) { return true; });
 }
 
 // compute_loop_las_hqs/resolve.cs:62-130
@@ -945,12 +949,14 @@ int launch_cull(const ViewParams& vp, const cr_batch* batches, int64_t nb, int64
                     capacity, quirks, scratch, list_cap < 0 ? nb : list_cap, (int32_t)node_slices);
 }
 
-template <int MODE, int PAYLOAD, int BLOCK, bool MANY, bool LIT>
-static int occupancy_list1() {
+// Resident CTAs per SM of an instance, asked for once (a driver query of its own
+// took 0.5 us of every frame).
+template <int MODE, int PAYLOAD, int BLOCK, int LIST, bool MANY, bool LIT>
+static int occupancy() {
     static const int n = [] {
         int k = 0;
         return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                   &k, k_batched<MODE, PAYLOAD, BLOCK, 1, MANY, LIT>, BLOCK, 0) == cudaSuccess && k > 0
+                   &k, k_batched<MODE, PAYLOAD, BLOCK, LIST, MANY, LIT>, BLOCK, 0) == cudaSuccess && k > 0
                    ? k
                    : 1;
     }();
@@ -966,7 +972,7 @@ static int launch_lists(const ViewParams& vp, const BatchedLaunch& bl, int grid,
     if (cudaGetDevice(&device) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
         return -1;
-    const int grid1 = std::min(grid, sms * occupancy_list1<MODE, PAYLOAD, BLOCK, MANY, LIT>());
+    const int grid1 = std::min(grid, sms * occupancy<MODE, PAYLOAD, BLOCK, 1, MANY, LIT>());
     PairParams pp;
     fill_pair_params(vp, &pp);
     if (launch_dep(k_batched<MODE, PAYLOAD, BLOCK, 1, MANY, LIT>, grid1, BLOCK, s, vp, bl, pp) != 0) return -1;
@@ -1003,23 +1009,13 @@ int launch_batched(const ViewParams& vp, const BatchedLaunch& bl, int block, int
 
 template <int MODE, int PAYLOAD>
 static int occupancy_t(int block, bool many, bool literal) {
-    int n = 0;
-    cudaError_t e;
-    if (literal) {
-        e = many ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_batched<MODE, PAYLOAD, 128, 0, true, true>, 128, 0)
-                 : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_batched<MODE, PAYLOAD, 128, 0, false, true>, 128, 0);
-        return e == cudaSuccess ? n : 1;
-    }
-    if (many) {
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_batched<MODE, PAYLOAD, 128, 0, true>, 128, 0);
-        return e == cudaSuccess ? n : 1;
-    }
+    if (literal) return many ? occupancy<MODE, PAYLOAD, 128, 0, true, true>() : occupancy<MODE, PAYLOAD, 128, 0, false, true>();
+    if (many) return occupancy<MODE, PAYLOAD, 128, 0, true, false>();
     switch (block) {
-        case 128: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_batched<MODE, PAYLOAD, 128, 0, false>, 128, 0); break;
-        case 512: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_batched<MODE, PAYLOAD, 512, 0, false>, 512, 0); break;
-        default: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_batched<MODE, PAYLOAD, 256, 0, false>, 256, 0); break;
+        case 128: return occupancy<MODE, PAYLOAD, 128, 0, false, false>();
+        case 512: return occupancy<MODE, PAYLOAD, 512, 0, false, false>();
+        default: return occupancy<MODE, PAYLOAD, 256, 0, false, false>();
     }
-    return e == cudaSuccess ? n : 1;
 }
 
 int batched_blocks_per_sm(int mode, int payload, int block, bool many, bool literal) {
@@ -1054,25 +1050,22 @@ int launch_plain(const float T[16], int32_t W, int32_t H, const cr_vertex* v, in
 int launch_resolve_index(int32_t W, int32_t H, uint64_t* fb, const uint32_t* rgba,
                          int64_t rgba_words, uint32_t* image, int clear_after, uint64_t clear,
                          void* stream, int tiles, uint32_t* scratch, uint32_t* counts) {
-    int64_t P = (int64_t)W * H, tail = (int64_t)W + 1;
-    int64_t threads = (P + 1) / 2 > tail ? (P + 1) / 2 : tail;
-    return launch_dep(k_resolve_index, blocks_for(threads, 256), 256, (cudaStream_t)stream, P, tail,
+    const int64_t P = (int64_t)W * H, tail = (int64_t)W + 1;
+    return launch_dep(k_resolve_index, blocks_for((P + 1) / 2, kPairs * kResolveBlock), kResolveBlock, (cudaStream_t)stream, P, tail,
                     fb, rgba, rgba_words, image, clear_after, clear, W, H, tiles, scratch, counts);
 }
 
 int launch_resolve_color(int32_t W, int32_t H, uint64_t* fb, uint32_t* image, int clear_after,
                          uint64_t clear, void* stream, uint32_t* scratch, uint32_t* counts) {
-    int64_t P = (int64_t)W * H, tail = (int64_t)W + 1;
-    int64_t threads = (P + 1) / 2 > tail ? (P + 1) / 2 : tail;
-    return launch_dep(k_resolve_color, blocks_for(threads, 256), 256, (cudaStream_t)stream, P, tail,
+    const int64_t P = (int64_t)W * H, tail = (int64_t)W + 1;
+    return launch_dep(k_resolve_color, blocks_for((P + 1) / 2, kPairs * kResolveBlock), kResolveBlock, (cudaStream_t)stream, P, tail,
                     fb, image, clear_after, clear, scratch, counts);
 }
 
 int launch_resolve_plain(int32_t W, int32_t H, uint64_t* fb, uint32_t* image, int clear_after,
                          uint64_t clear, int tiles, int zero_rule, void* stream) {
-    int64_t P = (int64_t)W * H, tail = (int64_t)W + 1;
-    int64_t threads = P > tail ? P : tail;
-    return launch_dep(k_resolve_plain, blocks_for(threads, 256), 256, (cudaStream_t)stream, P, tail,
+    const int64_t P = (int64_t)W * H, tail = (int64_t)W + 1;
+    return launch_dep(k_resolve_plain, blocks_for((P + 1) / 2, kPairs * kResolveBlock), kResolveBlock, (cudaStream_t)stream, P, tail,
                     W, H, tiles, zero_rule, fb, image, clear_after, clear);
 }
 

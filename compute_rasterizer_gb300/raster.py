@@ -51,6 +51,7 @@ class Context:
                           + self.lib.cr_status_string(st).decode())
         self.handle = h
         self.num_sms = self.lib.cr_ctx_num_sms(h)
+        self._cr_render = self.lib.cr_render  # looked up once: the call of every frame
 
     def close(self):
         if self.handle:
@@ -133,8 +134,10 @@ class Context:
     # ---- rendering ------------------------------------------------------------
     def render(self, cloud: "Cloud", view: L.View, params: L.RenderParams, fb: "Framebuffer",
                stream=None):
-        self.check(self.lib.cr_render(self.handle, cloud.handle, C.byref(view), C.byref(params),
-                                      fb.handle, stream), "cr_render")
+        st = self._cr_render(self.handle, cloud.handle, C.byref(view), C.byref(params), fb.handle,
+                             stream)
+        if st != L.OK:
+            self.check(st, "cr_render")
 
     def timing_enable(self, max_frames: int):
         self.check(self.lib.cr_timing_enable(self.handle, int(max_frames)), "timing enable")
