@@ -926,7 +926,7 @@ cr_status cr_render(cr_ctx* ctx, const cr_cloud* cloud, const cr_view* view,
                                                                  (quirks & CR_QUIRK_LITERAL_ARITH) != 0);
         if (per_sm < 1) per_sm = 1;
         const int grid = ctx->num_sms * per_sm;
-        if (launch_batched(vp, bl, block, grid, stream) != 0)
+        if (launch_batched(vp, bl, block, grid, stream, nb) != 0)
             return fail(ctx, CR_ERR_CUDA, "batched raster launch failed%s", "");
         mark(2 + pass, pass == 0 ? CR_STAGE_RASTER : CR_STAGE_HQS_COLOR);
     }

@@ -147,8 +147,9 @@ int launch_cull(const ViewParams& vp, const cr_batch* batches, int64_t nb_dispat
                 int64_t capacity, int32_t quirks, uint32_t* scratch, void* stream,
                 int64_t list_cap = -1, int node_slices = 0);
 // bl.quirks & CR_QUIRK_LITERAL_ARITH selects the literal instances (128 threads)
+// nb: batch records the cull looked at
 int launch_batched(const ViewParams& vp, const BatchedLaunch& bl, int block, int grid,
-                   void* stream);
+                   void* stream, int64_t nb);
 // variant 0: early-z, 1: dedup, 2: early-z & reduce (the three plain methods);
 // literal: CR_QUIRK_LITERAL_ARITH
 int launch_plain(const float T[16], int32_t W, int32_t H, const cr_vertex* v, int64_t n,

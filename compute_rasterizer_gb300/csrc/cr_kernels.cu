@@ -32,6 +32,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include "cr_internal.h"
 #include "cr_device.cuh"
@@ -482,9 +483,23 @@ __device__ __forceinline__ void run_points(const BatchedLaunch& bl, unsigned lon
 template <int MODE, int BLOCK, int LIST, bool UNCAPPED = false>
 constexpr int kMinBlocks = MODE != kModeHqsColor || UNCAPPED ? 0 : (LIST == 0 ? 9 : 8) * 128 / BLOCK;
 
+// How the pair uniforms reach an instance.  On 16 bytes the compiler reads them
+// two pairs at a time, which the index raster gains from (100M flight 795 -> 774
+// us, zoom 300M 440 -> 433) and the others lose by (1B points color 1320 -> 1350,
+// HQS 300M 1042 -> 1051).
+struct alignas(16) PairParams16 : PairParams {};
+template <int MODE, int PAYLOAD>
+using PairArg = std::conditional_t<MODE == kModeRaster && PAYLOAD == CR_PAYLOAD_INDEX, PairParams16, PairParams>;
+
+constexpr int64_t kOneGridBatches = 512;
+
 // LIST 0: the 10-bit items (front of the list region), LIST 1: the 20/30-bit
 // items (back of the region).  Each list runs in its own instance, so the
 // common 10-bit instance carries no wider decode state (fewer registers).
+// LIST 2: both lists in one grid, for clouds of at most kOneGridBatches batches,
+// whose frames are launches and latency: one launch less took the 50k preview
+// from 14.7 to 11.6 us; its registers (96 in the index raster) cost 1,500 batches
+// 9 % and the flight 10 %.
 // The frame's grids are programmatic dependents of one another, so a grid's
 // launch runs behind its predecessor's work (with the counter reset in the
 // resolve and the parallel file records: 50k points 21.3 -> 14.7 us, octree of 2M
@@ -501,19 +516,25 @@ constexpr int kMinBlocks = MODE != kModeHqsColor || UNCAPPED ? 0 : (LIST == 0 ? 
 // in [2^-64, 2^64]).
 template <int MODE, int PAYLOAD, int BLOCK, int LIST, bool MANY, bool LIT = false>
 __global__ void __launch_bounds__(BLOCK, (kMinBlocks<MODE, BLOCK, LIST, MANY && LIT>))
-    k_batched(ViewParams vp, BatchedLaunch bl, PairParams pp) {
-    if (LIST == 1) {
-        grid_wait();
-        grid_release();
-    }
+    k_batched(ViewParams vp, BatchedLaunch bl, PairArg<MODE, PAYLOAD> pp) {
+    if (LIST != 0) grid_wait();
+    if (LIST == 1) grid_release();
     __shared__ uint32_t s_item[2];
     __shared__ unsigned long long s_zc[MODE == kModeHqsColor ? 1 : kZCacheSlots];
-    uint32_t* cursor = bl.scratch + (LIST == 0 ? (MODE == kModeHqsColor ? kCursor1 : kCursor0)
+    uint32_t* cursor = bl.scratch + (LIST != 1 ? (MODE == kModeHqsColor ? kCursor1 : kCursor0)
                                                : (MODE == kModeHqsColor ? kCursor3 : kCursor2));
     const uint32_t nitems =
-        *reinterpret_cast<volatile uint32_t*>(bl.scratch + (LIST == 0 ? kItemCount : kItemCount2));
+        *reinterpret_cast<volatile uint32_t*>(bl.scratch + (LIST != 1 ? kItemCount : kItemCount2));
     const WorkSplit ws = split_work<BLOCK>(nitems, gridDim.x, bl.node_slices != 0);
-    if (blockIdx.x < ws.units) {
+    uint32_t units = ws.units;
+    // LIST 2 hands out the 20/30-bit list's units first
+    WorkSplit wide_ws;
+    if constexpr (LIST == 2) {
+        const uint32_t nwide = *reinterpret_cast<volatile uint32_t*>(bl.scratch + kItemCount2);
+        wide_ws = split_work<BLOCK>(nwide, gridDim.x, bl.node_slices != 0);
+        units += wide_ws.units;
+    }
+    if (blockIdx.x < units) {
         if (MODE != kModeHqsColor)
             for (int i = threadIdx.x; i < kZCacheSlots; i += BLOCK) s_zc[i] = kZCacheEmpty;
         // the first unit is the CTA's own number; the cursor hands out the rest
@@ -522,13 +543,20 @@ __global__ void __launch_bounds__(BLOCK, (kMinBlocks<MODE, BLOCK, LIST, MANY && 
         int buf = 0;
         while (true) {
             const uint32_t unit = s_item[buf];
-            if (unit >= ws.units) break;
+            if (unit >= units) break;
             if (threadIdx.x == 0) s_item[buf ^ 1] = gridDim.x + atomicAdd(cursor, 1u);
-            const Unit u = unit_range(ws, unit);
+            bool wide = LIST == 1;
+            Unit u;
+            if constexpr (LIST == 2) {
+                wide = unit < wide_ws.units;
+                u = wide ? unit_range(wide_ws, unit) : unit_range(ws, unit - wide_ws.units);
+            } else {
+                u = unit_range(ws, unit);
+            }
             const uint32_t wi = u.item;
             const int vb = u.vb, ve = u.ve;
             const uint32_t item = __ldcg(
-                bl.scratch + kScratchHead + (LIST == 0 ? (int64_t)wi : bl.list_cap - 1 - (int64_t)wi));
+                bl.scratch + kScratchHead + (wide ? bl.list_cap - 1 - (int64_t)wi : (int64_t)wi));
             const uint32_t b = item & (bl.node_slices ? kItemNodeMask : kItemBatchMask);
             const int level = (int)(item >> 29);  // levels 2-4 + kLevelInside: inside the view
 
@@ -567,7 +595,7 @@ __global__ void __launch_bounds__(BLOCK, (kMinBlocks<MODE, BLOCK, LIST, MANY && 
             // body without masks, other w-safe ones the pair body, the rest the
             // scalar body (see Body)
             const bool safe = (item & kItemWSafe) != 0;
-            if (LIST == 0 && safe && pair_batch_exact(c)) {
+            if (!wide && safe && pair_batch_exact(c)) {
                 if (level >= 2 + kLevelInside &&
                     (count == kPointsPerBatch ||
                      (kNodeSlice % (4 * BLOCK) == 0 && bl.node_slices && count == kNodeSlice)) &&
@@ -575,7 +603,7 @@ __global__ void __launch_bounds__(BLOCK, (kMinBlocks<MODE, BLOCK, LIST, MANY && 
                     run_points<MODE, PAYLOAD, BLOCK, 2, kBodyFull, LIT>(bl, s_zc, c, pp, first, count, l0_x12, vb, ve);
                 else
                     run_points<MODE, PAYLOAD, BLOCK, 2, kBodyPair, LIT>(bl, s_zc, c, pp, first, count, l0_x12, vb, ve);
-            } else if (LIST == 0) {
+            } else if (!wide) {
                 run_points<MODE, PAYLOAD, BLOCK, 2, kBodyScalar, LIT>(bl, s_zc, c, pp, first, count, l0_x12, vb, ve);
             } else if (level == 1) {
                 if (safe) run_points<MODE, PAYLOAD, BLOCK, 1, kBodyPair, LIT>(bl, s_zc, c, pp, first, count, l0_x12, vb, ve);
@@ -967,44 +995,50 @@ static int occupancy() {
 // then the 10-bit list as its programmatic dependent: it starts as soon as
 // every list-1 CTA has started, on the SM room list 1 leaves.
 template <int MODE, int PAYLOAD, int BLOCK, bool MANY, bool LIT = false>
-static int launch_lists(const ViewParams& vp, const BatchedLaunch& bl, int grid, cudaStream_t s) {
+static int launch_lists(const ViewParams& vp, const BatchedLaunch& bl, int grid, cudaStream_t s, int64_t nb) {
     int device = 0, sms = 1;
     if (cudaGetDevice(&device) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
         return -1;
-    const int grid1 = std::min(grid, sms * occupancy<MODE, PAYLOAD, BLOCK, 1, MANY, LIT>());
-    PairParams pp;
+    PairArg<MODE, PAYLOAD> pp;
     fill_pair_params(vp, &pp);
+    if constexpr (BLOCK == 128) {
+        if (nb <= kOneGridBatches)
+            return launch_dep(k_batched<MODE, PAYLOAD, BLOCK, 2, MANY, LIT>,
+                              std::min(grid, sms * occupancy<MODE, PAYLOAD, BLOCK, 2, MANY, LIT>()), BLOCK, s, vp, bl, pp);
+    }
+    const int grid1 = std::min(grid, sms * occupancy<MODE, PAYLOAD, BLOCK, 1, MANY, LIT>());
     if (launch_dep(k_batched<MODE, PAYLOAD, BLOCK, 1, MANY, LIT>, grid1, BLOCK, s, vp, bl, pp) != 0) return -1;
     return launch_dep(k_batched<MODE, PAYLOAD, BLOCK, 0, MANY, LIT>, grid, BLOCK, s, vp, bl, pp);
 }
 
 template <int MODE, int PAYLOAD>
 static int launch_batched_t(const ViewParams& vp, const BatchedLaunch& bl, int block, int grid,
-                            cudaStream_t s) {
+                            cudaStream_t s, int64_t nb) {
     // CR_QUIRK_LITERAL_ARITH, and clouds with more than kInlineFiles files:
     // 128-thread instances only
     if (bl.quirks & CR_QUIRK_LITERAL_ARITH) {
-        if (vp.nfiles > kInlineFiles) return launch_lists<MODE, PAYLOAD, 128, true, true>(vp, bl, grid, s);
-        return launch_lists<MODE, PAYLOAD, 128, false, true>(vp, bl, grid, s);
+        if (vp.nfiles > kInlineFiles) return launch_lists<MODE, PAYLOAD, 128, true, true>(vp, bl, grid, s, nb);
+        return launch_lists<MODE, PAYLOAD, 128, false, true>(vp, bl, grid, s, nb);
     }
-    if (vp.nfiles > kInlineFiles) return launch_lists<MODE, PAYLOAD, 128, true>(vp, bl, grid, s);
+    if (vp.nfiles > kInlineFiles) return launch_lists<MODE, PAYLOAD, 128, true>(vp, bl, grid, s, nb);
     switch (block) {
-        case 128: return launch_lists<MODE, PAYLOAD, 128, false>(vp, bl, grid, s);
-        case 512: return launch_lists<MODE, PAYLOAD, 512, false>(vp, bl, grid, s);
-        default: return launch_lists<MODE, PAYLOAD, 256, false>(vp, bl, grid, s);
+        case 128: return launch_lists<MODE, PAYLOAD, 128, false>(vp, bl, grid, s, nb);
+        case 512: return launch_lists<MODE, PAYLOAD, 512, false>(vp, bl, grid, s, nb);
+        default: return launch_lists<MODE, PAYLOAD, 256, false>(vp, bl, grid, s, nb);
     }
 }
 
-int launch_batched(const ViewParams& vp, const BatchedLaunch& bl, int block, int grid, void* stream) {
+int launch_batched(const ViewParams& vp, const BatchedLaunch& bl, int block, int grid, void* stream,
+                   int64_t nb) {
     cudaStream_t s = (cudaStream_t)stream;
     if (bl.mode == kModeRaster) {
         if (bl.payload == CR_PAYLOAD_COLOR)
-            return launch_batched_t<kModeRaster, CR_PAYLOAD_COLOR>(vp, bl, block, grid, s);
-        return launch_batched_t<kModeRaster, CR_PAYLOAD_INDEX>(vp, bl, block, grid, s);
+            return launch_batched_t<kModeRaster, CR_PAYLOAD_COLOR>(vp, bl, block, grid, s, nb);
+        return launch_batched_t<kModeRaster, CR_PAYLOAD_INDEX>(vp, bl, block, grid, s, nb);
     }
-    if (bl.mode == kModeHqsDepth) return launch_batched_t<kModeHqsDepth, CR_PAYLOAD_INDEX>(vp, bl, block, grid, s);
-    return launch_batched_t<kModeHqsColor, CR_PAYLOAD_INDEX>(vp, bl, block, grid, s);
+    if (bl.mode == kModeHqsDepth) return launch_batched_t<kModeHqsDepth, CR_PAYLOAD_INDEX>(vp, bl, block, grid, s, nb);
+    return launch_batched_t<kModeHqsColor, CR_PAYLOAD_INDEX>(vp, bl, block, grid, s, nb);
 }
 
 template <int MODE, int PAYLOAD>

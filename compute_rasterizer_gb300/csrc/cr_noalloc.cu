@@ -199,6 +199,6 @@ extern "C" cr_status cr_render_batched_noalloc(const cr_batch* d_batches, int64_
                                     : cr::batched_blocks_per_sm(bl.mode, bl.payload, block, many,
                                                                 literal != 0);
     if (per_sm < 1) per_sm = 1;
-    if (cr::launch_batched(vp, bl, block, sms * per_sm, stream) != 0) return CR_ERR_CUDA;
+    if (cr::launch_batched(vp, bl, block, sms * per_sm, stream, nb) != 0) return CR_ERR_CUDA;
     return CR_OK;
 }

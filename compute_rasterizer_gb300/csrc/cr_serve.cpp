@@ -334,7 +334,7 @@ cr_status enqueue(cr_server* s, Slot& sl, const CloudInfo& ci, const char** what
             const int block = c.plain_launches && c.block_threads > 0 ? c.block_threads : 128;
             const int per_sm = std::max(
                 1, cr::batched_blocks_per_sm(bl.mode, bl.payload, block, ci.nfiles > cr::kInlineFiles));
-            if (cr::launch_batched(vp, bl, block, s->num_sms * per_sm, sl.st) != 0) {
+            if (cr::launch_batched(vp, bl, block, s->num_sms * per_sm, sl.st, nb) != 0) {
                 *what = "plain raster launch";
                 return CR_ERR_CUDA;
             }

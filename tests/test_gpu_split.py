@@ -84,3 +84,36 @@ def test_multiview_item_counts(ctx, cloud_310, batches, block):
         mv.close()
     finally:
         cloud.set_loaded()
+
+
+# one grid for both lists up to 512 batches, two above; near the ground the cloud
+# has 20- and 30-bit batches beside 10-bit ones
+@pytest.mark.parametrize("batches", [511, 512, 513])
+@pytest.mark.parametrize("literal", [0, L.QUIRK_LITERAL_ARITH])
+def test_one_grid_or_two(ctx, batches, literal):
+    n = (batches - 1) * L.POINTS_PER_BATCH + 77
+    cl = encoded(n=n, extent=700.0, seed=batches)
+    cloud = ctx.cloud_from_arrays(cl["batches"], cl["lo"], cl["md"], cl["hi"], cl["rgba"],
+                                  cl["box_min"])
+    streams = (cl["lo"], cl["md"], cl["hi"], cl["rgba"])
+    for name in ("near", "mid"):
+        cam = cameras(cl, 321, 200)[name]
+        for method, payload in ((L.METHOD_LOOP_LAS, L.PAYLOAD_INDEX), (L.METHOD_LOOP_LAS, L.PAYLOAD_COLOR)):
+            fb, p = gpu_raw(ctx, cloud, cam, method, payload, quirks=QUIRKS[method] | literal)
+            with O.arith(O.ARITH_LITERAL if literal else O.ARITH_CONTRACT):
+                fr = oracle_frame(cam, cl["box_min"][None], QUIRKS[method], payload)
+                want = O.raster_batched(fr, cl["batches"], n, *streams)
+            got = fb.read(L.FB_WORDS)
+            assert np.array_equal(got, want), (name, payload, first_diff(got, want))
+            per_level = list(ctx.frame_stats(cloud, p).points_per_level)
+            assert per_level[1] > 0 and sum(per_level[2:]) > 0
+            fb.close()
+        q = QUIRKS[L.METHOD_LOOP_LAS_HQS]
+        fb, _ = gpu_raw(ctx, cloud, cam, L.METHOD_LOOP_LAS_HQS, quirks=q | literal)
+        with O.arith(O.ARITH_LITERAL if literal else O.ARITH_CONTRACT):
+            fr = oracle_frame(cam, cl["box_min"][None], q)
+            depth, accum, _ = O.hqs(fr, cl["batches"], n, *streams)
+        assert np.array_equal(fb.read(L.FB_DEPTH), depth)
+        assert np.array_equal(fb.read(L.FB_ACCUM), accum)
+        fb.close()
+    cloud.close()
