@@ -237,6 +237,38 @@ struct Emit<kModeRaster> {
     }
 };
 
+// The raster's candidates of a lane in 20/30-bit batches: the framebuffer words'
+// depths are read first, all four at once, and only a point that is not behind its
+// word issues the atomic.
+//
+// Those batches span hundreds of pixels, so lanes share none, the z-cache holds
+// little and the kernel is bound by the L2's 64-bit reductions (140 G/s, a read
+// costs half of one): unsorted 20M 135.7 -> 109.3 us, ground pose at 4K 82.8 ->
+// 73.6, octree of 2M 32.8 -> 29.1.  10-bit batches pass fewer points to the atomic
+// and lose by the read: with it at level 2 the 100M flight took 819 us, at levels 2
+// and 3 861, at all 939 (777 without).  In front of a single atomic, its latency
+// exposed, it measured slower everywhere.
+__device__ __forceinline__ void emit_read(const BatchedLaunch& bl, unsigned long long* zc, uint32_t bias,
+                                          bool ok[4], const uint32_t pix[4], const uint32_t wb[4],
+                                          const uint32_t pl[4]) {
+    unsigned long long* fb = reinterpret_cast<unsigned long long*>(bl.fb);
+    uint32_t depth[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        ok[j] = ok[j] && !zcache_rejects(zc, zslot_pixel(pix[j]), pix[j], wb[j]);
+        depth[j] = 0xFFFFFFFFu;
+        if (ok[j]) {
+            const uint32_t* high = reinterpret_cast<const uint32_t*>(fb + (pix[j] - bias)) + 1;
+            asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(depth[j]) : "l"(high) : "memory");
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+        if (ok[j] && wb[j] <= depth[j])
+            submit_min<unsigned long long>(fb + (pix[j] - bias), zc, zslot_pixel(pix[j]), pix[j],
+                                           ((unsigned long long)wb[j] << 32) | pl[j], wb[j]);
+}
+
 template <>
 struct Emit<kModeHqsDepth> {
     static __device__ __forceinline__ void run(const BatchedLaunch& bl, unsigned long long* zc,
@@ -469,8 +501,12 @@ __device__ __forceinline__ void run_points(const BatchedLaunch& bl, unsigned lon
             merge_pair<kTies>(0, 1, ok, pix, wb, pl);
             merge_pair<kTies>(2, 3, ok, pix, wb, pl);
             merge_pair<kTies>(0, 2, ok, pix, wb, pl);
+            if constexpr (MODE == kModeRaster && LC < 2) {
+                emit_read(bl, zc, bias, ok, pix, wb, pl);
+            } else {
 #pragma unroll
-            for (int j = 0; j < 4; j++) Emit<MODE>::run(bl, zc, bias, ok[j], pix[j], wb[j], pl[j]);
+                for (int j = 0; j < 4; j++) Emit<MODE>::run(bl, zc, bias, ok[j], pix[j], wb[j], pl[j]);
+            }
         }
     }
 }
