@@ -657,13 +657,16 @@ __global__ void __launch_bounds__(BLOCK, (kMinBlocks<MODE, BLOCK, LIST, MANY && 
 
 // ---- plain 16 B/point path --------------------------------------------------
 
+constexpr int kPlainSteps = 4;
+
 struct PlainParams {
     float T[16];
     int32_t W, H;
 };
 
 // VARIANT 0: compute_2021_earlyz/render.cs:35-74, key depth << 32 | color
-//   through the CTA z-cache.
+//   through the CTA z-cache, kPlainSteps points per thread with their loads in
+//   flight together.
 // VARIANT 1, 2: compute_2021_dedup/render.cs:33-69 and
 //   compute_2021_earlyz_reduce/render.cs:44-82.  A warp is 32 consecutive
 //   points (the grid stride is a multiple of 32), the reference's subgroup;
@@ -671,7 +674,8 @@ struct PlainParams {
 //   key = depth << 24 | color, the color's top byte overlapping the low depth
 //   byte as in the reference, so the reduction decides which keys reach the
 //   framebuffer.  Writers submit an atomicMin.
-template <int BLOCK, int VARIANT, bool LIT = false>
+// READ (VARIANT 0): the words' depths are read before the atomics (emit_read).
+template <int BLOCK, int VARIANT, bool LIT = false, bool READ = false>
 __global__ void __launch_bounds__(BLOCK) k_plain(PlainParams pp, const uint4* __restrict__ v,
                                                  int64_t n, uint64_t* __restrict__ fb) {
     grid_wait();
@@ -695,6 +699,33 @@ __global__ void __launch_bounds__(BLOCK) k_plain(PlainParams pp, const uint4* __
         __syncthreads();
     }
     uint32_t* warp_bits = s_bits + (VARIANT == 1 ? (threadIdx.x >> 5) * 128 : 0);
+    if constexpr (VARIANT == 0) {
+        constexpr int kTile = kPlainSteps * BLOCK;
+        for (int64_t base = (int64_t)blockIdx.x * kTile; base < n; base += (int64_t)gridDim.x * kTile) {
+            const int64_t i0 = base + threadIdx.x;
+            uint4 p[kPlainSteps];
+#pragma unroll
+            for (int k = 0; k < kPlainSteps; k++)
+                p[k] = i0 + k * BLOCK < n ? ld_stream(v + i0 + k * BLOCK) : make_uint4(0u, 0u, 0u, 0u);
+            bool ok[kPlainSteps];
+            uint32_t pix[kPlainSteps], wb[kPlainSteps], pl[kPlainSteps];
+#pragma unroll
+            for (int k = 0; k < kPlainSteps; k++) {
+                int32_t q;
+                ok[k] = project<false, LIT>(c, __uint_as_float(p[k].x), __uint_as_float(p[k].y),
+                                            __uint_as_float(p[k].z), q, wb[k]) && i0 + k * BLOCK < n;
+                pix[k] = (uint32_t)q;
+                pl[k] = p[k].w;
+            }
+            if constexpr (READ) {
+                emit_read(bl, s_zc, 0u, ok, pix, wb, pl);
+            } else {
+#pragma unroll
+                for (int k = 0; k < kPlainSteps; k++) Emit<kModeRaster>::run(bl, s_zc, 0u, ok[k], pix[k], wb[k], pl[k]);
+            }
+        }
+        return;
+    }
     const int64_t stride = (int64_t)gridDim.x * BLOCK;
     for (int64_t base = (int64_t)blockIdx.x * BLOCK; base < n; base += stride) {
         const int64_t i = base + threadIdx.x;
@@ -705,10 +736,6 @@ __global__ void __launch_bounds__(BLOCK) k_plain(PlainParams pp, const uint4* __
         uint32_t wbits;
         const bool ok = project<false, LIT>(c, __uint_as_float(p.x), __uint_as_float(p.y),
                                             __uint_as_float(p.z), pix, wbits) && act;
-        if (VARIANT == 0) {
-            Emit<kModeRaster>::run(bl, s_zc, 0u, ok, (uint32_t)pix, wbits, p.w);
-            continue;
-        }
         // wbits = floatBitsToInt(pos.w), positive for every point in view
         bool write;
         if (VARIANT == 1) {
@@ -1103,18 +1130,26 @@ int launch_plain(const float T[16], int32_t W, int32_t H, const cr_vertex* v, in
     for (int i = 0; i < 16; i++) pp.T[i] = T[i];
     pp.W = W;
     pp.H = H;
-    int64_t need = (n + 255) / 256;
-    if (need < grid) grid = (int)need;
+    // A point whose word is read first spares the L2 a reduction where it lies behind
+    // (a read costs half of one), and waits for the read where it does not: from
+    // about 5 points per pixel on, given enough of them to hide the wait.  Read first
+    // against not, us per frame at 1920x1080: 4 points per pixel 65.6 / 64.8, 5 77.8 /
+    // 80.4, 8 104 / 122, 31 307 / 435; at 640x640 8 (3.3M points) 29.8 / 26.1, 16
+    // (6.5M) 49.0 / 52.4; 16M at 256x256 104 / 178.
+    const bool read = variant == 0 && n >= 6000000 && n >= 5 * (int64_t)W * H;
+    const int per = 256 * (variant == 0 ? kPlainSteps : 1);
+    grid = (int)std::min<int64_t>((n + per - 1) / per, grid);
     const uint4* v4 = reinterpret_cast<const uint4*>(v);
     cudaStream_t s = (cudaStream_t)stream;
+    const auto launch = [&](auto* k) { return launch_dep(k, grid, 256, s, pp, v4, n, fb); };
     if (literal) {
-        if (variant == 1) return launch_dep(k_plain<256, 1, true>, grid, 256, s, pp, v4, n, fb);
-        if (variant == 2) return launch_dep(k_plain<256, 2, true>, grid, 256, s, pp, v4, n, fb);
-        return launch_dep(k_plain<256, 0, true>, grid, 256, s, pp, v4, n, fb);
+        if (variant == 1) return launch(k_plain<256, 1, true>);
+        if (variant == 2) return launch(k_plain<256, 2, true>);
+        return read ? launch(k_plain<256, 0, true, true>) : launch(k_plain<256, 0, true>);
     }
-    if (variant == 1) return launch_dep(k_plain<256, 1>, grid, 256, s, pp, v4, n, fb);
-    if (variant == 2) return launch_dep(k_plain<256, 2>, grid, 256, s, pp, v4, n, fb);
-    return launch_dep(k_plain<256, 0>, grid, 256, s, pp, v4, n, fb);
+    if (variant == 1) return launch(k_plain<256, 1>);
+    if (variant == 2) return launch(k_plain<256, 2>);
+    return read ? launch(k_plain<256, 0, false, true>) : launch(k_plain<256, 0>);
 }
 
 int launch_resolve_index(int32_t W, int32_t H, uint64_t* fb, const uint32_t* rgba,
