@@ -360,7 +360,7 @@ __device__ __forceinline__ void wait_tile() {
     __syncthreads();
 }
 
-// A tile kernel's dynamic shared memory, allowed once per kernel and process.
+// A tile kernel's dynamic shared memory, allowed on the current device.
 template <typename K>
 bool allow_shared(K kernel, int bytes) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
@@ -417,34 +417,54 @@ __global__ void __launch_bounds__(512, 2) k_morton_keys(MortonFrame f, const uin
 // Finishes a radix sort that left out the keys' lowest `low` bits: each run of
 // equal upper bits, in index order so far, is insertion-sorted by the whole key
 // (stable, so ties keep the index order).  Runs longer than kMaxRun raise *flag
-// and stay.  One thread per run; a run's neighbours compare upper bits only, which
-// no swap inside a run changes.
-constexpr int kMaxRun = 64;
+// and stay.  One thread per run, in the CTA of the run's first key: the keys of a
+// tile, the key before and kMaxRun after it come to shared memory first (sorting
+// in global memory left a thread's dependent loads in a row: 40M keys 250 us, now
+// 208).  A
+// run that moved is written back whole; the neighbouring CTA, which has its last
+// keys too, takes only their upper bits, which no move changes.
+constexpr int kMaxRun = 64, kRunTile = 1024;
 __global__ void __launch_bounds__(256) k_sort_runs(unsigned long long* keys, uint32_t* idx, int64_t n, int low,
                                                    uint32_t* flag) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n - 1;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const unsigned long long head = keys[i] >> low;
-        if (keys[i + 1] >> low != head || (i > 0 && keys[i - 1] >> low == head)) continue;
-        int len = 2;
-        while (i + len < n && len <= kMaxRun && keys[i + len] >> low == head) len++;
-        if (len > kMaxRun) {
-            *flag = 1u;
-            continue;
+    __shared__ unsigned long long s_key[1 + kRunTile + kMaxRun];
+    __shared__ uint32_t s_idx[1 + kRunTile + kMaxRun];
+    for (int64_t base = (int64_t)blockIdx.x * kRunTile; base < n; base += (int64_t)gridDim.x * kRunTile) {
+        const int cnt = (int)min((int64_t)(kRunTile + kMaxRun), n - base);  // keys from base on
+        for (int k = (int)threadIdx.x - (base > 0); k < cnt; k += 256) {
+            s_key[1 + k] = keys[base + k];
+            s_idx[1 + k] = idx[base + k];
         }
-        for (int k = 1; k < len; k++) {
-            const unsigned long long key = keys[i + k];
-            const uint32_t id = idx[i + k];
-            int j = k;
-            for (; j > 0 && keys[i + j - 1] > key; j--) {
-                keys[i + j] = keys[i + j - 1];
-                idx[i + j] = idx[i + j - 1];
+        __syncthreads();
+        for (int i = 1 + threadIdx.x; i < 1 + min(cnt, kRunTile); i += 256) {
+            const unsigned long long head = s_key[i] >> low;
+            if (i == cnt || s_key[i + 1] >> low != head || ((i > 1 || base > 0) && s_key[i - 1] >> low == head)) continue;
+            int len = 2;
+            while (len <= kMaxRun && i + len <= cnt && s_key[i + len] >> low == head) len++;
+            // (a run of exactly kMaxRun may end with the copy: counted as too long)
+            if (len >= kMaxRun) {
+                *flag = 1u;
+                continue;
             }
-            if (j != k) {
-                keys[i + j] = key;
-                idx[i + j] = id;
+            bool moved = false;
+            for (int k = 1; k < len; k++) {
+                const unsigned long long key = s_key[i + k];
+                const uint32_t id = s_idx[i + k];
+                int j = k;
+                for (; j > 0 && s_key[i + j - 1] > key; j--) {
+                    s_key[i + j] = s_key[i + j - 1];
+                    s_idx[i + j] = s_idx[i + j - 1];
+                }
+                s_key[i + j] = key;
+                s_idx[i + j] = id;
+                moved = moved || j != k;
+            }
+            if (!moved) continue;
+            for (int k = 0; k < len; k++) {
+                keys[base + i - 1 + k] = s_key[i + k];
+                idx[base + i - 1 + k] = s_idx[i + k];
             }
         }
+        __syncthreads();
     }
 }
 
@@ -674,13 +694,11 @@ __global__ void __launch_bounds__(S::kThreads, S::kCtas) k_encode(EncodeArgs a, 
 template <typename S>
 cudaError_t launch_encode(const EncodeArgs& a, const uint8_t* rec, cr_batch* batches, uint32_t* lo, uint32_t* md,
                           uint32_t* hi, uint32_t* rgba, unsigned nb, cudaStream_t s) {
-    static const bool allowed = allow_shared(k_encode<true, S>, S::kShared) && allow_shared(k_encode<false, S>, S::kShared);
-    if (!allowed) return cudaErrorInvalidConfiguration;
     const int tile = tile_records(a.bpp, S::kBytes);
-    if ((a.bpp & 1) == 0 && (a.rgb < 0 || (a.rgb & 1) == 0))
-        k_encode<true, S><<<nb, S::kThreads, S::kShared, s>>>(a, rec, tile, batches, lo, md, hi, rgba);
-    else
-        k_encode<false, S><<<nb, S::kThreads, S::kShared, s>>>(a, rec, tile, batches, lo, md, hi, rgba);
+    const bool even = (a.bpp & 1) == 0 && (a.rgb < 0 || (a.rgb & 1) == 0);
+    const auto kernel = even ? k_encode<true, S> : k_encode<false, S>;
+    if (!allow_shared(kernel, S::kShared)) return cudaErrorInvalidConfiguration;
+    kernel<<<nb, S::kThreads, S::kShared, s>>>(a, rec, tile, batches, lo, md, hi, rgba);
     return cudaGetLastError();
 }
 
@@ -878,8 +896,9 @@ cr_status cr_morton_sort_device(cr_ctx* ctx, uint8_t* d_rec, int64_t n, int32_t 
     // took 2 ms of a 40M-point sort in the driver): keys and indices twice, the
     // radix sort's own, a copy of the records (the gather reads it and writes d_rec
     // in place), a flag.
-    const cudaMemPool_t pool = cr::ctx_pool(ctx);
-    if (!pool) return CR_ERR_CUDA;
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return CR_ERR_CUDA;
+    const cudaMemPool_t pool = device == cr::ctx_device(ctx) ? cr::ctx_pool(ctx) : nullptr;
     cub::DoubleBuffer<unsigned long long> keys;
     cub::DoubleBuffer<uint32_t> vals;
     size_t cub_bytes = 0;
@@ -888,9 +907,8 @@ cr_status cr_morton_sort_device(cr_ctx* ctx, uint8_t* d_rec, int64_t n, int32_t 
     const auto padded = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
     const size_t key_bytes = padded((size_t)n * 8), val_bytes = padded((size_t)n * 4);
     uint8_t* buf = nullptr;
-    e = cudaMallocFromPoolAsync(
-        reinterpret_cast<void**>(&buf),
-        2 * key_bytes + 2 * val_bytes + padded(cub_bytes) + padded((size_t)n * bpp) + 256, pool, s);
+    const size_t bytes = 2 * key_bytes + 2 * val_bytes + padded(cub_bytes) + padded((size_t)n * bpp) + 256;
+    e = pool ? cudaMallocFromPoolAsync(reinterpret_cast<void**>(&buf), bytes, pool, s) : cudaMalloc(&buf, bytes);
     if (e != cudaSuccess) return cuda_status(e);
     uint8_t* at = buf;
     const auto take = [&at](size_t bytes) {
@@ -906,8 +924,7 @@ cr_status cr_morton_sort_device(cr_ctx* ctx, uint8_t* d_rec, int64_t n, int32_t 
     // tiles start on 16 bytes: records that do not are copied to where they do first
     const bool aligned = (reinterpret_cast<uintptr_t>(d_rec) & 15) == 0;
     if (!aligned) e = cudaMemcpyAsync(copy, d_rec, (size_t)n * bpp, cudaMemcpyDeviceToDevice, s);
-    static const bool tiles = allow_shared(k_morton_keys, 2 * kTileBytes);
-    if (e == cudaSuccess && !tiles) e = cudaErrorInvalidConfiguration;
+    if (e == cudaSuccess && !allow_shared(k_morton_keys, 2 * kTileBytes)) e = cudaErrorInvalidConfiguration;
     if (e == cudaSuccess) {
         const int tile = tile_records(bpp, kTileBytes);  // bpp <= kGatherMaxBpp: at least 832
         const int grid = (int)std::min<int64_t>((n + tile - 1) / tile, 2 * (int64_t)cr_ctx_num_sms(ctx));
@@ -926,7 +943,7 @@ cr_status cr_morton_sort_device(cr_ctx* ctx, uint8_t* d_rec, int64_t n, int32_t 
     if (e == cudaSuccess)
         e = cub::DeviceRadixSort::SortPairs(cub_tmp, cub_bytes, keys, vals, (int)n, low, 63, s);
     if (e == cudaSuccess) {
-        k_sort_runs<<<grid_for(n), 256, 0, s>>>(keys.Current(), vals.Current(), n, low, flag);
+        k_sort_runs<<<(unsigned)std::min<int64_t>((n + kRunTile - 1) / kRunTile, 65535), 256, 0, s>>>(keys.Current(), vals.Current(), n, low, flag);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(&long_runs, flag, 4, cudaMemcpyDeviceToHost, s);
@@ -940,7 +957,7 @@ cr_status cr_morton_sort_device(cr_ctx* ctx, uint8_t* d_rec, int64_t n, int32_t 
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    cudaFreeAsync(buf, s);
+    pool ? cudaFreeAsync(buf, s) : cudaFree(buf);
     return cuda_status(e);
 }
 
