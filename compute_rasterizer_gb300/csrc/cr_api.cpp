@@ -11,6 +11,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <string>
 #include <vector>
@@ -38,7 +39,10 @@ struct cr_ctx {
     // leaves them so; one without a resolve, or that failed on the way, does not
     bool counters_zero = false;
     bool captured = false;  // a frame was captured into a graph
-    cudaMemPool_t pool = nullptr;  // ctx_pool
+    // WorkBuffer: the kept buffer, and whether a call holds it
+    std::mutex work_mutex;
+    uint8_t* work = nullptr;
+    size_t work_bytes = 0;
     std::vector<cr_frame_events> timing;  // GLTimerQueries-style event pairs
     int32_t timing_used = 0;
     std::string last_error;
@@ -255,20 +259,28 @@ int cr::default_quirks_for(int32_t method) { return default_quirks(method); }
 
 int cr::ctx_device(const cr_ctx* ctx) { return ctx ? ctx->device : 0; }
 
-cudaMemPool_t cr::ctx_pool(cr_ctx* ctx) {
-    if (ctx->pool) return ctx->pool;
-    cudaMemPoolProps props = {};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = ctx->device;
-    cudaMemPool_t pool = nullptr;
-    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) return nullptr;
-    uint64_t keep = kPoolKeepBytes;
-    if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
-        cudaMemPoolDestroy(pool);
-        return nullptr;
+cr::WorkBuffer::WorkBuffer(cr_ctx* ctx, size_t bytes) {
+    int device = 0;
+    status = cudaGetDevice(&device);
+    if (status != cudaSuccess) return;
+    if (bytes > kKeepBytes || device != ctx->device || !ctx->work_mutex.try_lock()) {
+        status = cudaMalloc(&data, bytes);
+        return;
     }
-    return ctx->pool = pool;
+    held_ = ctx;
+    if (ctx->work_bytes < bytes) {
+        if (ctx->work) cudaFree(ctx->work);
+        ctx->work = nullptr;
+        ctx->work_bytes = 0;
+        status = cudaMalloc(&ctx->work, bytes);
+        if (status == cudaSuccess) ctx->work_bytes = bytes;
+    }
+    data = ctx->work;
+}
+
+cr::WorkBuffer::~WorkBuffer() {
+    if (held_) held_->work_mutex.unlock();
+    else if (data) cudaFree(data);
 }
 
 cr_status cr::view_params_for(const cr_view* view, const double* box_min, int32_t num_files,
@@ -405,7 +417,7 @@ cr_status cr_ctx_destroy(cr_ctx* ctx) {
     destroy_timing(ctx);
     if (ctx->scratch) cudaFree(ctx->scratch);
     if (ctx->files) cudaFree(ctx->files);
-    if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
+    if (ctx->work) cudaFree(ctx->work);
     delete ctx;
     return CR_OK;
 }

@@ -213,11 +213,23 @@ cr_status encode_records_device(const uint8_t* d_rec, int64_t n, int32_t bpp, in
                                 uint32_t* d_lo, uint32_t* d_md, uint32_t* d_hi, uint32_t* d_rgba,
                                 void* stream);
 int ctx_device(const cr_ctx* ctx);
-// The context's pool of device memory for builders' temporary buffers, created on
-// first use; null if that fails.  Between uses it keeps up to kPoolKeepBytes, and
-// nothing once the context is destroyed.
-constexpr uint64_t kPoolKeepBytes = 4ull << 30;
-cudaMemPool_t ctx_pool(cr_ctx* ctx);
+// Device memory for one builder call, whose stream is idle when it is given back.
+// Up to kKeepBytes come from a buffer that the context keeps (and frees when it is
+// destroyed) and one call at a time holds; a larger or a second one, or one on
+// another device than the context's, is allocated and freed.
+constexpr size_t kKeepBytes = (size_t)4 << 30;
+class WorkBuffer {
+  public:
+    WorkBuffer(cr_ctx* ctx, size_t bytes);
+    ~WorkBuffer();
+    WorkBuffer(const WorkBuffer&) = delete;
+    WorkBuffer& operator=(const WorkBuffer&) = delete;
+    uint8_t* data = nullptr;
+    cudaError_t status = cudaSuccess;
+
+  private:
+    cr_ctx* held_ = nullptr;  // the context whose buffer this is
+};
 
 // ---- multi-view frames (cr_multiview.cu), shared by cr_mv plans and the server
 

@@ -892,13 +892,9 @@ cr_status cr_morton_sort_device(cr_ctx* ctx, uint8_t* d_rec, int64_t n, int32_t 
     if (n <= 1) return CR_OK;
     cudaStream_t s = (cudaStream_t)stream;
     const MortonFrame f = morton_frame(hdr);
-    // The sort's buffers in one allocation of the context's pool (six of their own
-    // took 2 ms of a 40M-point sort in the driver): keys and indices twice, the
-    // radix sort's own, a copy of the records (the gather reads it and writes d_rec
-    // in place), a flag.
-    int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess) return CR_ERR_CUDA;
-    const cudaMemPool_t pool = device == cr::ctx_device(ctx) ? cr::ctx_pool(ctx) : nullptr;
+    // The sort's buffers in one piece (six allocations of their own took 2 ms of a
+    // 40M-point sort in the driver): keys and indices twice, the radix sort's own, a
+    // copy of the records (the gather reads it and writes d_rec in place), a flag.
     cub::DoubleBuffer<unsigned long long> keys;
     cub::DoubleBuffer<uint32_t> vals;
     size_t cub_bytes = 0;
@@ -906,11 +902,9 @@ cr_status cr_morton_sort_device(cr_ctx* ctx, uint8_t* d_rec, int64_t n, int32_t 
     if (e != cudaSuccess) return cuda_status(e);
     const auto padded = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
     const size_t key_bytes = padded((size_t)n * 8), val_bytes = padded((size_t)n * 4);
-    uint8_t* buf = nullptr;
-    const size_t bytes = 2 * key_bytes + 2 * val_bytes + padded(cub_bytes) + padded((size_t)n * bpp) + 256;
-    e = pool ? cudaMallocFromPoolAsync(reinterpret_cast<void**>(&buf), bytes, pool, s) : cudaMalloc(&buf, bytes);
-    if (e != cudaSuccess) return cuda_status(e);
-    uint8_t* at = buf;
+    cr::WorkBuffer buf(ctx, 2 * key_bytes + 2 * val_bytes + padded(cub_bytes) + padded((size_t)n * bpp) + 256);
+    if (buf.status != cudaSuccess) return cuda_status(buf.status);
+    uint8_t* at = buf.data;
     const auto take = [&at](size_t bytes) {
         uint8_t* p = at;
         at += bytes;
@@ -956,9 +950,9 @@ cr_status cr_morton_sort_device(cr_ctx* ctx, uint8_t* d_rec, int64_t n, int32_t 
         k_gather<<<grid, 32 * kGatherWarps, 0, s>>>(copy, d_rec, vals.Current(), n, bpp, aligned);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    pool ? cudaFreeAsync(buf, s) : cudaFree(buf);
-    return cuda_status(e);
+    // idle before the buffer is given back, after an error too
+    const cudaError_t done = cudaStreamSynchronize(s);
+    return cuda_status(e == cudaSuccess ? done : e);
 }
 
 cr_status cr_encode_las_device(cr_ctx* ctx, const uint8_t* d_rec, int64_t n, int32_t bpp, int32_t fmt,
