@@ -354,8 +354,9 @@ struct Emit;
 // the key's depth as the word's upper bound in the cache: after the atomic the
 // word holds at most `key`.  A cache miss goes straight to the atomic (a
 // fire-and-forget RED): reading the word first to skip the atomic for a point
-// behind it measured 4 % slower on the single-view raster and 9 % on the
-// multi-view one, the read's latency costing more than the extra REDs.
+// behind it measured slower at 10 bit, on the single-view raster and the
+// multi-view one (the callers that read first do so for four words at once, see
+// emit_read).
 template <typename T>
 __device__ __forceinline__ void submit_min(T* g, unsigned long long* zc, uint32_t slot,
                                            uint32_t tag, T key, uint32_t depth_of_key) {
