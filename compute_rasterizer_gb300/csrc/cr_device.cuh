@@ -7,6 +7,7 @@
 
 #include <cstdint>
 
+#include "cr_inside.h"
 #include "cr_internal.h"
 
 namespace cr {
@@ -135,32 +136,6 @@ __device__ __forceinline__ bool w_safe(const float* T, float mnx, float mny, flo
     }
     const float err = fmul(mag, 0x1p-16f);
     return fsub(lo, err) >= lo_bound && fadd(hi, err) <= hi_bound;
-}
-
-// Whether every point decoded from a batch that w_safe() passed projects inside
-// the view (|x / w| <= 1 and |y / w| <= 1): w - |x| and w - |y| are minima of
-// linear functions, so over the AABB they are least at corners.  The margin,
-// 2^-15 of the term sums of both rows, is far above the rounding of the two
-// rows (see w_safe) and of the quotient (2^-22 of w).
-__device__ __forceinline__ bool all_inside(const float* T, float mnx, float mny, float mnz, float mxx,
-                                           float mxy, float mxz) {
-    float slack = 0.0f, mag = 0.0f;
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-        const float x = (k & 1) ? mxx : mnx, y = (k & 2) ? mxy : mny, z = (k & 4) ? mxz : mnz;
-        float p[3], m[3];
-#pragma unroll
-        for (int r = 0; r < 3; r++) {
-            const int c = r == 2 ? 3 : r;
-            p[r] = __fmaf_rn(T[8 + c], z, __fmaf_rn(T[4 + c], y, __fmaf_rn(T[c], x, T[12 + c])));
-            m[r] = fadd(fadd(fadd(fabsf(fmul(T[c], x)), fabsf(fmul(T[4 + c], y))),
-                             fabsf(fmul(T[8 + c], z))), fabsf(T[12 + c]));
-        }
-        const float s = fsub(p[2], fmaxf(fabsf(p[0]), fabsf(p[1])));
-        slack = k == 0 ? s : fminf(slack, s);
-        mag = fmaxf(mag, fadd(fadd(m[0], m[1]), m[2]));
-    }
-    return slack >= fmul(mag, 0x1p-15f);
 }
 
 // ---- per-batch math (render.cs:130-231), no contraction --------------------
