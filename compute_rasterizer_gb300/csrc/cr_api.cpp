@@ -34,7 +34,6 @@ struct cr_ctx {
     int64_t last_dispatched = 0;  // batch records the last cull looked at
     int64_t last_list_cap = 0;    // words of its item-list region
     bool last_node_slices = false;
-    bool last_resolved = false;
     // whether the next frame finds the counters at zero: a frame's resolve
     // leaves them so; one without a resolve, or that failed on the way, does not
     bool counters_zero = false;
@@ -892,15 +891,15 @@ cr_status cr_render(cr_ctx* ctx, const cr_cloud* cloud, const cr_view* view,
     ctx->last_dispatched = nb;
     ctx->last_list_cap = list_cap;
     ctx->last_node_slices = slices;
-    ctx->last_resolved = p->resolve != 0;
 
     // a captured frame runs at times this host code does not see, so it, and every
-    // frame after it, zeroes the counters itself
+    // frame after it, zeroes the counters itself; so does a frame without batches,
+    // which launches no cull to clear kResolved
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (st != nullptr && st != cudaStreamLegacy &&
         (cudaStreamIsCapturing(st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone))
         ctx->captured = true;
-    if (!ctx->counters_zero || ctx->captured)
+    if (!ctx->counters_zero || ctx->captured || nb <= 0)
         CR_CUDA(ctx, cudaMemsetAsync(ctx->scratch, 0, kCounterWords * 4, st), "counter reset");
     ctx->counters_zero = false;
     if (launch_cull(vp, cloud->batches, nb, cloud->capacity, quirks, ctx->scratch, stream, list_cap,
@@ -956,12 +955,14 @@ cr_status cr_last_frame_stats(cr_ctx* ctx, const cr_cloud* cloud, const cr_rende
     if (!ctx || !cloud || !p || !out || cloud->plain) return CR_ERR_INVALID_ARG;
     std::memset(out, 0, sizeof(*out));
     CR_CUDA(ctx, cudaDeviceSynchronize(), "synchronize");
-    // counts of a frame without a resolve are still where the cull counted
-    uint32_t counts[kCounterWords] = {};
-    CR_CUDA(ctx, cudaMemcpy(counts, ctx->last_resolved ? frame_counts(ctx) : ctx->scratch,
-                            (ctx->last_resolved ? 2 : kCounterWords) * 4, cudaMemcpyDeviceToHost),
+    uint32_t head[kCounterWords] = {}, counts[2] = {};
+    CR_CUDA(ctx, cudaMemcpy(head, ctx->scratch, sizeof(head), cudaMemcpyDeviceToHost), "count read");
+    CR_CUDA(ctx, cudaMemcpy(counts, frame_counts(ctx), sizeof(counts), cudaMemcpyDeviceToHost),
             "count read");
-    const uint32_t n_front = counts[kItemCount], n_back = counts[ctx->last_resolved ? 1 : kItemCount2];
+    const uint32_t n_front = head[kResolved] ? counts[0] : head[kItemCount];
+    const uint32_t n_back = head[kResolved] ? counts[1] : head[kItemCount2];
+    if ((int64_t)n_front + n_back > ctx->last_list_cap)  // a graph of a larger cloud's frame ran last
+        return fail(ctx, CR_ERR_INVALID_ARG, "the last frame was another cloud's%s", "");
     const uint32_t count = n_front + n_back;
     std::vector<uint32_t> items(count);
     if (n_front)

@@ -109,7 +109,8 @@ enum : int {
     kItemCount2 = 3,  // items in the 20/30-bit list
     kCursor2 = 4,     // dynamic work cursor, 20/30-bit list, raster / HQS depth pass
     kCursor3 = 5,     // dynamic work cursor, 20/30-bit list, HQS color pass
-    kCounterWords = 6,
+    kResolved = 6,    // 1: the frame's resolve has moved the item counts (finish_lists)
+    kCounterWords = 7,
     kErrWord = 7,     // sticky device error bits (cleared by cr_ctx_check)
     kScratchHead = 8  // item lists start here
 };
@@ -156,7 +157,7 @@ int launch_plain(const float T[16], int32_t W, int32_t H, const cr_vertex* v, in
                  uint64_t* fb, int grid, int variant, void* stream, int literal = 0);
 // tiles: CR_QUIRK_RESOLVE_TILES (image words outside full 16x16 tiles kept).
 // scratch (the batched resolves): zero its counters, their two item counts kept
-// in counts[0], counts[1]
+// in counts[0], counts[1], and set kResolved
 int launch_resolve_index(int32_t W, int32_t H, uint64_t* fb, const uint32_t* rgba,
                          int64_t rgba_words, uint32_t* image, int clear_after, uint64_t clear,
                          void* stream, int tiles = 0, uint32_t* scratch = nullptr,

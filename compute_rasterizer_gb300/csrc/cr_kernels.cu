@@ -131,6 +131,7 @@ __global__ void __launch_bounds__(256) k_cull(const __grid_constant__ ViewParams
                                               int32_t node_slices) {
     grid_wait();
     int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (b == 0) scratch[kResolved] = 0u;
     bool keep = false;
     uint32_t item = 0, slices = 1;
     if (b < nb) {
@@ -789,12 +790,13 @@ __global__ void __launch_bounds__(BLOCK) k_plain(PlainParams pp, const uint4* __
 // The frame's list counters, reset for the next frame's cull by the resolve that
 // follows the last raster pass (a reset of its own in front of the cull cost
 // 1.8 us per frame; one by the raster's last CTA 4-40 % of the raster).  The two
-// item counts stay in `counts` for cr_last_frame_stats.
+// item counts stay in `counts` for cr_last_frame_stats, which kResolved tells where
+// they are: with graphs replayed, only the device knows which frame ran last.
 __device__ __forceinline__ void finish_lists(uint32_t* scratch, uint32_t* counts) {
     if (!scratch || blockIdx.x != 0 || threadIdx.x != 0) return;
     counts[0] = scratch[kItemCount];
     counts[1] = scratch[kItemCount2];
-    for (int k = 0; k < kCounterWords; k++) scratch[k] = 0u;
+    for (int k = 0; k < kCounterWords; k++) scratch[k] = k == kResolved ? 1u : 0u;
 }
 
 __device__ __forceinline__ bool depth_valid(uint64_t v) {
