@@ -415,56 +415,51 @@ __global__ void __launch_bounds__(512, 2) k_morton_keys(MortonFrame f, const uin
 }
 
 // Finishes a radix sort that left out the keys' lowest `low` bits: each run of
-// equal upper bits, in index order so far, is insertion-sorted by the whole key
-// (stable, so ties keep the index order).  Runs longer than kMaxRun raise *flag
-// and stay.  One thread per run, in the CTA of the run's first key: the keys of a
-// tile, the key before and kMaxRun after it come to shared memory first (sorting
-// in global memory left a thread's dependent loads in a row: 40M keys 250 us, now
-// 208).  A
-// run that moved is written back whole; the neighbouring CTA, which has its last
-// keys too, takes only their upper bits, which no move changes.
+// equal upper bits, in index order so far, is sorted by the whole key (stable, so
+// ties keep the index order).  A run of kMaxRun keys raises *flag, and the rest of the
+// work is left, for the caller then sorts by all bits.  The keys of a
+// tile, the key before and kMaxRun after it come to shared memory; each key finds
+// its place by counting, in its run, the larger ones before it and the smaller ones
+// after it, so a run is the work of as many threads as it has keys (an insertion
+// sort by one thread per run was as fast on runs of one or two keys, but a sort of
+// 5M points whose header spans 30 times their extent took 1712 us, now 1171, and
+// one of 40M at 10 times 13.3 ms, now 6.6; 1.2 and 6.8 with passes over all bits).
+// A run belongs to the CTA of its first key, which writes the keys that moved; the
+// neighbouring CTA, which has its last keys too, takes only their upper bits, which
+// no move changes.
 constexpr int kMaxRun = 64, kRunTile = 1024;
 __global__ void __launch_bounds__(256) k_sort_runs(unsigned long long* keys, uint32_t* idx, int64_t n, int low,
                                                    uint32_t* flag) {
     __shared__ unsigned long long s_key[1 + kRunTile + kMaxRun];
     __shared__ uint32_t s_idx[1 + kRunTile + kMaxRun];
     for (int64_t base = (int64_t)blockIdx.x * kRunTile; base < n; base += (int64_t)gridDim.x * kRunTile) {
+        // (also the barrier between one tile's last reads and the next one's copy)
+        if (__syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<volatile uint32_t*>(flag))) return;
         const int cnt = (int)min((int64_t)(kRunTile + kMaxRun), n - base);  // keys from base on
-        for (int k = (int)threadIdx.x - (base > 0); k < cnt; k += 256) {
+        const int before = base > 0 ? 1 : 0;
+        for (int k = (int)threadIdx.x - before; k < cnt; k += 256) {
             s_key[1 + k] = keys[base + k];
             s_idx[1 + k] = idx[base + k];
         }
         __syncthreads();
-        for (int i = 1 + threadIdx.x; i < 1 + min(cnt, kRunTile); i += 256) {
-            const unsigned long long head = s_key[i] >> low;
-            if (i == cnt || s_key[i + 1] >> low != head || ((i > 1 || base > 0) && s_key[i - 1] >> low == head)) continue;
-            int len = 2;
-            while (len <= kMaxRun && i + len <= cnt && s_key[i + len] >> low == head) len++;
-            // (a run of exactly kMaxRun may end with the copy: counted as too long)
-            if (len >= kMaxRun) {
-                *flag = 1u;
+        for (int i = 1 + threadIdx.x; i <= cnt; i += 256) {
+            const unsigned long long key = s_key[i], head = key >> low;
+            // first..last: the run, as far as the copy and kMaxRun keys each way go
+            int first = i, last = i, at = i;
+            while (first > 1 - before && i - first < kMaxRun && s_key[first - 1] >> low == head)
+                at -= s_key[--first] > key;
+            // begins before or after the tile, or is too long
+            if (first < 1 || first > kRunTile || i - first >= kMaxRun) continue;
+            while (last < cnt && last - first < kMaxRun && s_key[last + 1] >> low == head)
+                at += s_key[++last] < key;
+            if (last - first + 1 >= kMaxRun) {  // (may go on past the copy)
+                if (i == first) *flag = 1u;
                 continue;
             }
-            bool moved = false;
-            for (int k = 1; k < len; k++) {
-                const unsigned long long key = s_key[i + k];
-                const uint32_t id = s_idx[i + k];
-                int j = k;
-                for (; j > 0 && s_key[i + j - 1] > key; j--) {
-                    s_key[i + j] = s_key[i + j - 1];
-                    s_idx[i + j] = s_idx[i + j - 1];
-                }
-                s_key[i + j] = key;
-                s_idx[i + j] = id;
-                moved = moved || j != k;
-            }
-            if (!moved) continue;
-            for (int k = 0; k < len; k++) {
-                keys[base + i - 1 + k] = s_key[i + k];
-                idx[base + i - 1 + k] = s_idx[i + k];
-            }
+            if (at == i) continue;
+            keys[base + at - 1] = key;
+            idx[base + at - 1] = s_idx[i];
         }
-        __syncthreads();
     }
 }
 
@@ -927,23 +922,32 @@ cr_status cr_morton_sort_device(cr_ctx* ctx, uint8_t* d_rec, int64_t n, int32_t 
         e = cudaGetLastError();
     }
     // Radix passes over the upper 40 bits (48 above 2^26 points), 5 (6) in place of 8
-    // at 0.3 ms each for 40M points; k_sort_runs (0.1 ms) finishes the runs they leave
-    // equal.  A surface scan fills about two bits of three, so 40 bits are 2^26
-    // cells and runs stay short; points so clustered that a run passes kMaxRun get
-    // the passes over all bits after all.
-    const int low = n <= ((int64_t)1 << 26) ? 23 : 15;
-    uint32_t long_runs = 0;
-    if (e == cudaSuccess) e = cudaMemsetAsync(flag, 0, 4, s);
+    // at 0.3 ms each for 40M points; k_sort_runs (0.2 ms) finishes the runs they leave
+    // equal.  A surface scan fills about two bits of three, so 40 bits are 2^26 cells
+    // and runs stay short; points so clustered that a run reaches kMaxRun (a far
+    // outlier stretches the header's cube, or duplicates) get the passes over all bits
+    // after all.  The sort then takes, against all bits at once with allocations of
+    // its own: 40M points 6.1-6.6 ms (6.7-6.9), 5M 0.99-1.17 (1.2), 300k 302 us (495).
+    // Up to kFullKeys points, where it would lose (80,000 points 280 us against 245,
+    // 10,000 335 against 145), all bits come first and only: 131 us at 10,000 points,
+    // 166 at 65,536 (115 and 145 by the short passes, where no run is long).
+    constexpr int64_t kFullKeys = 8 * cr::kPointsPerBatch;
+    const int low = n <= kFullKeys ? 0 : n <= ((int64_t)1 << 26) ? 23 : 15;
     if (e == cudaSuccess)
         e = cub::DeviceRadixSort::SortPairs(cub_tmp, cub_bytes, keys, vals, (int)n, low, 63, s);
-    if (e == cudaSuccess) {
-        k_sort_runs<<<(unsigned)std::min<int64_t>((n + kRunTile - 1) / kRunTile, 65535), 256, 0, s>>>(keys.Current(), vals.Current(), n, low, flag);
-        e = cudaGetLastError();
+    if (low > 0) {
+        uint32_t long_runs = 0;
+        if (e == cudaSuccess) e = cudaMemsetAsync(flag, 0, 4, s);
+        if (e == cudaSuccess) {
+            k_sort_runs<<<(unsigned)std::min<int64_t>((n + kRunTile - 1) / kRunTile, 65535), 256, 0, s>>>(
+                keys.Current(), vals.Current(), n, low, flag);
+            e = cudaGetLastError();
+        }
+        if (e == cudaSuccess) e = cudaMemcpyAsync(&long_runs, flag, 4, cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e == cudaSuccess && long_runs)
+            e = cub::DeviceRadixSort::SortPairs(cub_tmp, cub_bytes, keys, vals, (int)n, 0, 63, s);
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&long_runs, flag, 4, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e == cudaSuccess && long_runs)
-        e = cub::DeviceRadixSort::SortPairs(cub_tmp, cub_bytes, keys, vals, (int)n, 0, 63, s);
     if (e == cudaSuccess) {
         const int64_t warps = (n + 31) / 32;
         const int grid = (int)std::min<int64_t>((warps + kGatherWarps - 1) / kGatherWarps, 65535);
