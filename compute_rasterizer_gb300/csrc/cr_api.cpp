@@ -148,7 +148,7 @@ cr_status enqueue_file_records(cr_ctx* ctx, const cr_cloud* cloud, const cr_view
             ctx->files = nullptr;
             ctx->files_cap = 0;
         }
-        CR_CUDA(ctx, cudaMalloc(&ctx->files, sizeof(FileRec) * (size_t)cloud->nfiles), "file records");
+        CR_CUDA(ctx, ctx_alloc(ctx, &ctx->files, sizeof(FileRec) * (size_t)cloud->nfiles), "file records");
         ctx->files_cap = cloud->nfiles;
     }
     if (launch_file_records(view->view, view->proj, cloud->box_min.data(), cloud->nfiles, ctx->files,
@@ -178,7 +178,7 @@ cr_status ensure_scratch(cr_ctx* ctx, int64_t items) {
         ctx->scratch_words = 0;
     }
     int64_t words = std::max<int64_t>(need, 1 << 16);
-    CR_CUDA(ctx, cudaMalloc(&ctx->scratch, words * 4), "scratch allocation");
+    CR_CUDA(ctx, ctx_alloc(ctx, &ctx->scratch, words * 4), "scratch allocation");
     CR_CUDA(ctx, cudaMemset(ctx->scratch, 0, words * 4), "scratch clear");
     ctx->scratch_words = words;
     ctx->counters_zero = false;  // cleared on another stream than the frame's, perhaps
@@ -262,8 +262,9 @@ cr::WorkBuffer::WorkBuffer(cr_ctx* ctx, size_t bytes) {
     int device = 0;
     status = cudaGetDevice(&device);
     if (status != cudaSuccess) return;
+    if (bytes > kKeepBytes) release_work(ctx);
     if (bytes > kKeepBytes || device != ctx->device || !ctx->work_mutex.try_lock()) {
-        status = cudaMalloc(&data, bytes);
+        status = ctx_alloc(ctx, &data, bytes);
         return;
     }
     held_ = ctx;
@@ -280,6 +281,25 @@ cr::WorkBuffer::WorkBuffer(cr_ctx* ctx, size_t bytes) {
 cr::WorkBuffer::~WorkBuffer() {
     if (held_) held_->work_mutex.unlock();
     else if (data) cudaFree(data);
+}
+
+bool cr::release_work(cr_ctx* ctx) {
+    std::unique_lock<std::mutex> lock(ctx->work_mutex, std::try_to_lock);
+    if (!lock.owns_lock() || !ctx->work) return false;
+    cudaFree(ctx->work);
+    ctx->work = nullptr;
+    ctx->work_bytes = 0;
+    return true;
+}
+
+cudaError_t cr::ctx_alloc(cr_ctx* ctx, void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    for (int again = 0; e == cudaErrorMemoryAllocation && again < 2; again++) {
+        cudaGetLastError();  // the caller reports it: none is left for the process's next check
+        if (again == 1 || !release_work(ctx)) break;
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
 }
 
 cr_status cr::view_params_for(const cr_view* view, const double* box_min, int32_t num_files,
@@ -477,11 +497,11 @@ cr_status cr_cloud_create(cr_ctx* ctx, int64_t n, int64_t nb, int32_t nfiles, in
     uint32_t** streams[4] = {&c->lo, &c->md, &c->hi, &c->rgba};
     for (int i = 0; i < 4 && e == cudaSuccess; i++) {
         if (!(mask & (1 << i))) continue;
-        e = cudaMalloc(streams[i], bytes);
+        e = ctx_alloc(ctx, streams[i], bytes);
         if (e == cudaSuccess) e = cudaMemset(*streams[i], 0, bytes);
     }
     if (e == cudaSuccess && nb > 0) {
-        e = cudaMalloc(&c->batches, (size_t)nb * sizeof(cr_batch));
+        e = ctx_alloc(ctx, &c->batches, (size_t)nb * sizeof(cr_batch));
         if (e == cudaSuccess) e = cudaMemset(c->batches, 0, (size_t)nb * sizeof(cr_batch));
     }
     if (e != cudaSuccess) {
@@ -651,7 +671,7 @@ cr_status cr_cloud_create_plain(cr_ctx* ctx, int64_t n, cr_cloud** out) {
     c->n = n;
     c->nfiles = 1;
     c->box_min.assign(3, 0.0);
-    cudaError_t e = cudaMalloc(&c->verts, (size_t)std::max<int64_t>(n, 1) * sizeof(cr_vertex));
+    cudaError_t e = ctx_alloc(ctx, &c->verts, (size_t)std::max<int64_t>(n, 1) * sizeof(cr_vertex));
     if (e != cudaSuccess) {
         delete c;
         return cuda_fail(ctx, e, "plain cloud allocation");
@@ -688,12 +708,12 @@ cr_status cr_fb_create(cr_ctx* ctx, int32_t W, int32_t H, int32_t kind, cr_fb** 
     f->words = (int64_t)W * H + W + 1;
     cudaError_t e;
     if (kind == CR_FB_U64) {
-        e = cudaMalloc(&f->fb, (size_t)f->words * 8);
+        e = ctx_alloc(ctx, &f->fb, (size_t)f->words * 8);
     } else {
-        e = cudaMalloc(&f->depth, (size_t)f->words * 4);
-        if (e == cudaSuccess) e = cudaMalloc(&f->accum, (size_t)f->words * 16);
+        e = ctx_alloc(ctx, &f->depth, (size_t)f->words * 4);
+        if (e == cudaSuccess) e = ctx_alloc(ctx, &f->accum, (size_t)f->words * 16);
     }
-    if (e == cudaSuccess) e = cudaMalloc(&f->image, (size_t)W * H * 4);
+    if (e == cudaSuccess) e = ctx_alloc(ctx, &f->image, (size_t)W * H * 4);
     // a new image starts at zero: pixels a resolve does not cover (the plain
     // methods' partial tiles) read back as 0, not as stale device memory
     if (e == cudaSuccess) e = cudaMemset(f->image, 0, (size_t)W * H * 4);

@@ -215,9 +215,10 @@ cr_status encode_records_device(const uint8_t* d_rec, int64_t n, int32_t bpp, in
                                 void* stream);
 int ctx_device(const cr_ctx* ctx);
 // Device memory for one builder call, whose stream is idle when it is given back.
-// Up to kKeepBytes come from a buffer that the context keeps (and frees when it is
-// destroyed) and one call at a time holds; a larger or a second one, or one on
-// another device than the context's, is allocated and freed.
+// Up to kKeepBytes come from a buffer that the context keeps and one call at a time
+// holds; a larger or a second one, or one on another device than the context's, is
+// allocated and freed.  The kept buffer is freed with the context, before a larger
+// one is allocated, and by release_work.
 constexpr size_t kKeepBytes = (size_t)4 << 30;
 class WorkBuffer {
   public:
@@ -231,6 +232,14 @@ class WorkBuffer {
   private:
     cr_ctx* held_ = nullptr;  // the context whose buffer this is
 };
+// Frees the context's kept buffer unless a call holds it; whether it did.
+bool release_work(cr_ctx* ctx);
+// cudaMalloc; where memory has run out, once more without the kept buffer.
+cudaError_t ctx_alloc(cr_ctx* ctx, void** p, size_t bytes);
+template <typename T>
+cudaError_t ctx_alloc(cr_ctx* ctx, T** p, size_t bytes) {
+    return ctx_alloc(ctx, reinterpret_cast<void**>(p), bytes);
+}
 
 // ---- multi-view frames (cr_multiview.cu), shared by cr_mv plans and the server
 

@@ -78,7 +78,7 @@ cr_status cr_cloud_load_las(cr_ctx* ctx, cr_cloud* cloud, const void* records, i
     const int64_t bpp = info->bytes_per_point;
     const int64_t task = CR_MAX_POINTS_PER_LOAD;
     uint8_t* staging = nullptr;
-    if (cudaMalloc(&staging, (size_t)(std::min(n, task) * bpp)) != cudaSuccess) {
+    if (cr::ctx_alloc(ctx, &staging, (size_t)(std::min(n, task) * bpp)) != cudaSuccess) {
         cudaGetLastError();
         return CR_ERR_OUT_OF_MEMORY;
     }

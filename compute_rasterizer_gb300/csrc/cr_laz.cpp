@@ -1813,7 +1813,7 @@ cr_status cr_cloud_load_laz(cr_ctx* ctx, cr_cloud* cloud, const cr_laz* laz, int
     uint8_t* staging = nullptr;
     cudaEvent_t copied[3] = {nullptr, nullptr, nullptr};
     cudaStream_t st = (cudaStream_t)stream;
-    cudaError_t e = cudaMalloc(&staging, (size_t)(window * bpp));
+    cudaError_t e = cr::ctx_alloc(ctx, &staging, (size_t)(window * bpp));
     for (int r = 0; r < R && e == cudaSuccess; r++) {
         e = cudaHostAlloc(&host[r], (size_t)(window * bpp), cudaHostAllocDefault);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&copied[r], cudaEventDisableTiming);

@@ -953,14 +953,14 @@ cr_status cr_mv_create(cr_ctx* ctx, const cr_cloud* cloud, int32_t nviews, const
         delete mv;
         return s;
     }
-    cudaError_t e = cudaMalloc(&mv->fbs, words * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&mv->images, std::max<int64_t>(pixels, 1) * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&mv->d_views, sizeof(MVView) * nviews);
-    if (e == cudaSuccess) e = cudaMalloc(&mv->d_files, sizeof(MVFile) * (size_t)nviews * mv->ci.nfiles);
-    if (e == cudaSuccess) e = cudaMalloc(&mv->scratch, mv_scratch_words(mv->ci.nb_total, nviews) * 4);
+    cudaError_t e = cr::ctx_alloc(ctx, &mv->fbs, words * 8);
+    if (e == cudaSuccess) e = cr::ctx_alloc(ctx, &mv->images, std::max<int64_t>(pixels, 1) * 4);
+    if (e == cudaSuccess) e = cr::ctx_alloc(ctx, &mv->d_views, sizeof(MVView) * nviews);
+    if (e == cudaSuccess) e = cr::ctx_alloc(ctx, &mv->d_files, sizeof(MVFile) * (size_t)nviews * mv->ci.nfiles);
+    if (e == cudaSuccess) e = cr::ctx_alloc(ctx, &mv->scratch, mv_scratch_words(mv->ci.nb_total, nviews) * 4);
     if (e == cudaSuccess) e = cudaMemset(mv->scratch, 0, mv_scratch_words(mv->ci.nb_total, nviews) * 4);
     if (e == cudaSuccess) e = cudaHostAlloc(&mv->h_views, sizeof(MVView) * nviews, cudaHostAllocDefault);
-    if (e == cudaSuccess) e = cudaMalloc(&mv->d_pairs, sizeof(uint32_t) * nviews);
+    if (e == cudaSuccess) e = cr::ctx_alloc(ctx, &mv->d_pairs, sizeof(uint32_t) * nviews);
     if (e == cudaSuccess) e = cudaHostAlloc(&mv->h_pairs, sizeof(uint32_t) * nviews, cudaHostAllocDefault);
     if (e == cudaSuccess) {
         std::memset(mv->h_pairs, 0, sizeof(uint32_t) * nviews);
@@ -971,8 +971,8 @@ cr_status cr_mv_create(cr_ctx* ctx, const cr_cloud* cloud, int32_t nviews, const
             e = cudaHostAlloc(&mv->h_files, sizeof(MVFile) * (size_t)nviews * mv->ci.nfiles,
                               cudaHostAllocDefault);
     } else {
-        if (e == cudaSuccess) e = cudaMalloc(&mv->d_mats, sizeof(double) * 32 * (size_t)nviews);
-        if (e == cudaSuccess) e = cudaMalloc(&mv->d_box, sizeof(double) * 3 * (size_t)mv->ci.nfiles);
+        if (e == cudaSuccess) e = cr::ctx_alloc(ctx, &mv->d_mats, sizeof(double) * 32 * (size_t)nviews);
+        if (e == cudaSuccess) e = cr::ctx_alloc(ctx, &mv->d_box, sizeof(double) * 3 * (size_t)mv->ci.nfiles);
         if (e == cudaSuccess)
             e = cudaHostAlloc(&mv->h_mats, sizeof(double) * 32 * (size_t)nviews, cudaHostAllocDefault);
         if (e == cudaSuccess)

@@ -598,6 +598,7 @@ cr_status cr_server_create(cr_ctx* ctx, const cr_server_config* cfg, cr_server**
         delete s;
         return CR_ERR_CUDA;
     }
+    cr::release_work(ctx);  // the slots' buffers grow later, without the context
     cudaError_t e = cudaMalloc(&s->pool, c.pool_bytes);
     s->alloc.init(c.pool_bytes);
     s->slots.resize(c.max_inflight);

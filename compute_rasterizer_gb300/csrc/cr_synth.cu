@@ -860,7 +860,7 @@ cr_status cr_synth_points_device(cr_ctx* ctx, const cr_synth_params* p, int64_t 
     cudaStream_t s = (cudaStream_t)stream;
     int32_t init[6] = {INT32_MAX, INT32_MAX, INT32_MAX, INT32_MIN, INT32_MIN, INT32_MIN};
     int32_t* d_mm = nullptr;
-    cudaError_t e = cudaMalloc(&d_mm, sizeof(init));
+    cudaError_t e = cr::ctx_alloc(ctx, &d_mm, sizeof(init));
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_mm, init, sizeof(init), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess && n > 0) {
         k_gen<<<grid_for(n) * 4 > 65535 ? 65535 : grid_for(n) * 4, 256, 0, s>>>(*p, 1.0 / p->las_scale,
@@ -884,6 +884,7 @@ cr_status cr_morton_sort_device(cr_ctx* ctx, uint8_t* d_rec, int64_t n, int32_t 
     if (!ctx || n < 0 || (n > 0 && !d_rec) || bpp < 12 || (bpp & 1) || bpp > kGatherMaxBpp || !hdr ||
         n >= ((int64_t)1 << 31))
         return CR_ERR_INVALID_ARG;
+    if (n == 0) cr::release_work(ctx);
     if (n <= 1) return CR_OK;
     cudaStream_t s = (cudaStream_t)stream;
     const MortonFrame f = morton_frame(hdr);
@@ -981,7 +982,7 @@ cr_status cr_synth_cloud_device(cr_ctx* ctx, const cr_synth_params* p, int64_t n
     cr_status st = cr_cloud_device(cloud, &db, &lo, &md, &hi, &rgba);
     if (st != CR_OK || !lo || !md || !hi || !rgba) return CR_ERR_INVALID_ARG;
     uint8_t* rec = nullptr;
-    cudaError_t e = cudaMalloc(&rec, (size_t)n * kRecBytes);
+    cudaError_t e = cr::ctx_alloc(ctx, &rec, (size_t)n * kRecBytes);
     if (e != cudaSuccess) return cuda_status(e);
     st = cr_synth_points_device(ctx, p, n, rec, hdr, stream);
     if (st == CR_OK) st = cr_morton_sort_device(ctx, rec, n, kRecBytes, hdr, stream);

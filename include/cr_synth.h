@@ -67,7 +67,11 @@ cr_status cr_morton_sort_host(uint8_t* records, int64_t n, int32_t bytes_per_poi
 cr_status cr_synth_points_device(cr_ctx* ctx, const cr_synth_params* p, int64_t n,
                                  uint8_t* d_records, cr_las_header* hdr, void* stream);
 /* Device Morton sort (stable radix sort of (code, index), then a gather);
- * records of an even bytes_per_point in [12, 64], as LAS point formats are. */
+ * records of an even bytes_per_point in [12, 64], as LAS point formats are.
+ * The context keeps the sort's buffers for the next call, up to 4 GB (about
+ * 54 bytes per point of format 2).  It frees them when an allocation of its own
+ * runs out of memory, when a call needs more, with n = 0 (which sorts nothing),
+ * when a server is created, and in cr_ctx_destroy. */
 cr_status cr_morton_sort_device(cr_ctx* ctx, uint8_t* d_records, int64_t n,
                                 int32_t bytes_per_point, const cr_las_header* hdr, void* stream);
 /* GPU encoder: loadLas (LasLoaderSparse.cpp:37-212) over device records, one
