@@ -9,6 +9,7 @@
 
 #include "cr_inside.h"
 #include "cr_internal.h"
+#include "cr_occupancy.h"
 
 namespace cr {
 namespace {
@@ -40,6 +41,17 @@ int launch_dep(void (*k)(KArgs...), dim3 grid, dim3 block, cudaStream_t s, Args&
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, k, static_cast<Args&&>(args)...) == cudaSuccess ? 0 : -1;
+}
+
+// Resident CTAs of `k` per SM of the current device (cr_occupancy.h).
+template <typename K>
+int kernel_occupancy(OccupancyCache& cache, K k, int block) {
+    int device = -1;
+    if (cudaGetDevice(&device) != cudaSuccess) return 1;
+    return cached_occupancy(cache, device, [=] {
+        int n = 0;
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, block, 0) == cudaSuccess ? n : 0;
+    });
 }
 
 // Waits until the grids this one depends on have finished and their writes are

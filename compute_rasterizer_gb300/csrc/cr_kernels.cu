@@ -1042,18 +1042,11 @@ int launch_cull(const ViewParams& vp, const cr_batch* batches, int64_t nb, int64
                     capacity, quirks, scratch, list_cap < 0 ? nb : list_cap, (int32_t)node_slices);
 }
 
-// Resident CTAs per SM of an instance, asked for once (a driver query of its own
-// took 0.5 us of every frame).
+// Resident CTAs per SM of an instance.
 template <int MODE, int PAYLOAD, int BLOCK, int LIST, bool MANY, bool LIT>
 static int occupancy() {
-    static const int n = [] {
-        int k = 0;
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                   &k, k_batched<MODE, PAYLOAD, BLOCK, LIST, MANY, LIT>, BLOCK, 0) == cudaSuccess && k > 0
-                   ? k
-                   : 1;
-    }();
-    return n;
+    static OccupancyCache cache;
+    return kernel_occupancy(cache, k_batched<MODE, PAYLOAD, BLOCK, LIST, MANY, LIT>, BLOCK);
 }
 
 // The (usually short) 20/30-bit list with a grid that is resident at once,

@@ -598,17 +598,11 @@ __global__ void k_mv_fill_views(const MVView* __restrict__ views, unsigned long 
         fb[i] = v;
 }
 
-// The 10-bit list, then the 20/30-bit list, on one stream.
+// Resident CTAs per SM of the list-1 instance.
 template <int PAYLOAD, int BLOCK>
 int mv_occupancy_list1() {
-    static const int n = [] {
-        int k = 0;
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, k_mv_raster<PAYLOAD, BLOCK, 1>, BLOCK,
-                                                             0) == cudaSuccess && k > 0
-                   ? k
-                   : 1;
-    }();
-    return n;
+    static OccupancyCache cache;
+    return kernel_occupancy(cache, k_mv_raster<PAYLOAD, BLOCK, 1>, BLOCK);
 }
 
 // The 20/30-bit list with a grid that is resident at once, then the 10-bit
