@@ -512,13 +512,23 @@ __device__ __forceinline__ void run_points(const BatchedLaunch& bl, unsigned lon
     }
 }
 
-// Resident CTAs per SM of the HQS color pass: 9 for the 10-bit list (56
-// registers; HQS 300M 1067 us, against 1077 at 10 CTAs, where the masked pair
-// body spills, and 1069 at 8), 8 for the 20/30-bit list (uncapped it takes 90
-// registers, 5 CTAs).  UNCAPPED: the many-file literal instance, which spills
-// under the cap.
-template <int MODE, int BLOCK, int LIST, bool UNCAPPED = false>
-constexpr int kMinBlocks = MODE != kModeHqsColor || UNCAPPED ? 0 : (LIST == 0 ? 9 : 8) * 128 / BLOCK;
+// Resident CTAs per SM that the compiler is held to in the HQS color pass (128
+// threads; bytes of spill stores and registers from ptxas).
+//   10-bit list: 9 (no spill, 54; HQS 300M 1067 us, against 1077 at 10 CTAs, where
+//   the masked pair body spills, and 1069 at 8); literal 8 (no spill, 62; 100M zoom
+//   513 us, against 524 at 9 CTAs and 64 bytes of spills).
+//   20/30-bit list: 6 (no spill, 70; many files 5, where 6 spill; 10M unsorted points
+//   223 us, 40M ground at 4K 173, against 238 and 178 at 8 CTAs, 88 bytes).
+//   both lists in one grid: 5 (52 bytes, literal 148; 96).  50k points zoom / ground
+//   25.2 / 24.1 us, 1M 43.7 / 30.8, 2.3M 66.1 / 42.4; at 8 CTAs (392-492 bytes) 26.9 /
+//   25.5, 43.9 / 33.2, 67.3 / 44.6; uncapped (no spill, 112) 24.6 / 23.6, but 1M zoom
+//   45.5 and 2.5M 62.9 against 59.4.
+// The many-file literal instances of the single lists take 71 and 96 registers
+// uncapped, 12 bytes, and spill more under a cap.
+template <int MODE, int BLOCK, int LIST, bool MANY, bool LIT>
+constexpr int kMinBlocks = MODE != kModeHqsColor || (MANY && LIT && LIST != 2)
+                               ? 0
+                               : (LIST == 0 ? (LIT ? 8 : 9) : (LIST == 1 && !MANY ? 6 : 5)) * 128 / BLOCK;
 
 // How the pair uniforms reach an instance.  On 16 bytes the compiler reads them
 // two pairs at a time, which the index raster gains from (100M flight 795 -> 774
@@ -528,7 +538,12 @@ struct alignas(16) PairParams16 : PairParams {};
 template <int MODE, int PAYLOAD>
 using PairArg = std::conditional_t<MODE == kModeRaster && PAYLOAD == CR_PAYLOAD_INDEX, PairParams16, PairParams>;
 
-constexpr int64_t kOneGridBatches = 512;
+// Batches up to which a pass draws both lists in one grid (LIST 2, below).  The HQS
+// color pass, whose one grid holds fewer CTAs, gains by it up to about 224 batches:
+// 2.3M points zoom / ground 66.1 / 42.4 us in one grid, 63.4 / 46.2 in two; 2.6M 70.9 /
+// 44.7 and 65.7 / 47.6; 3.5M 84.0 / 47.8 and 70.7 / 50.1; 50k 25.2 / 24.1 and 28.4 / 26.8.
+template <int MODE>
+constexpr int64_t kOneGridBatches = MODE == kModeHqsColor ? 224 : 512;
 
 // LIST 0: the 10-bit items (front of the list region), LIST 1: the 20/30-bit
 // items (back of the region).  Each list runs in its own instance, so the
@@ -552,7 +567,7 @@ constexpr int64_t kOneGridBatches = 512;
 // them (the pairs with project_pair10's literal body, on batches whose w lies
 // in [2^-64, 2^64]).
 template <int MODE, int PAYLOAD, int BLOCK, int LIST, bool MANY, bool LIT = false>
-__global__ void __launch_bounds__(BLOCK, (kMinBlocks<MODE, BLOCK, LIST, MANY && LIT>))
+__global__ void __launch_bounds__(BLOCK, (kMinBlocks<MODE, BLOCK, LIST, MANY, LIT>))
     k_batched(ViewParams vp, BatchedLaunch bl, PairArg<MODE, PAYLOAD> pp) {
     if (LIST != 0) grid_wait();
     if (LIST == 1) grid_release();
@@ -1061,7 +1076,7 @@ static int launch_lists(const ViewParams& vp, const BatchedLaunch& bl, int grid,
     PairArg<MODE, PAYLOAD> pp;
     fill_pair_params(vp, &pp);
     if constexpr (BLOCK == 128) {
-        if (nb <= kOneGridBatches)
+        if (nb <= kOneGridBatches<MODE>)
             return launch_dep(k_batched<MODE, PAYLOAD, BLOCK, 2, MANY, LIT>,
                               std::min(grid, sms * occupancy<MODE, PAYLOAD, BLOCK, 2, MANY, LIT>()), BLOCK, s, vp, bl, pp);
     }

@@ -521,8 +521,15 @@ __device__ __forceinline__ void mv_raster_items(const MVArgs& a) {
 // cull, then lets the list-0 grid start at once; every list-0 CTA waits for the
 // list-1 grid before it exits, so the resolve that follows sees both lists'
 // writes.
+// Held to 8 CTAs of 128 threads per SM (64 registers, no spill) in list 0: 64 views of
+// 200M points 6829 us, against 6952 at 7 CTAs.  CTAs of 64 threads spill there and are
+// held to 14 of the 16 (50M points 404 against 410 us).  List 1 takes 113-122 registers
+// uncapped; held to 5 CTAs it spilled 32-96 bytes and was no faster (66.3 / 365 / 3998 us
+// inside clouds of 2M, 20M and 200M points, 65.3 / 365 / 3990 uncapped).
+template <int BLOCK, int LIST>
+constexpr int kMvMinBlocks = LIST == 1 ? 0 : (BLOCK == 64 ? 14 : 8 * 128 / BLOCK);
 template <int PAYLOAD, int BLOCK, int LIST>
-__global__ void __launch_bounds__(BLOCK, (LIST == 0 ? 8 : 5) * 128 / BLOCK) k_mv_raster(MVArgs a) {
+__global__ void __launch_bounds__(BLOCK, (kMvMinBlocks<BLOCK, LIST>)) k_mv_raster(MVArgs a) {
     if (LIST == 1) {
         grid_wait();
         grid_release();
