@@ -524,11 +524,13 @@ __device__ __forceinline__ void run_points(const BatchedLaunch& bl, unsigned lon
 //   25.5, 43.9 / 33.2, 67.3 / 44.6; uncapped (no spill, 112) 24.6 / 23.6, but 1M zoom
 //   45.5 and 2.5M 62.9 against 59.4.
 // The many-file literal instances of the single lists take 71 and 96 registers
-// uncapped, 12 bytes, and spill more under a cap.
+// uncapped, 12 bytes, and spill more under a cap.  Wider CTAs: as many threads, for
+// the 20/30-bit list rounded up (512 threads, 40M ground: 2 CTAs 95 us, 1 99).
 template <int MODE, int BLOCK, int LIST, bool MANY, bool LIT>
 constexpr int kMinBlocks = MODE != kModeHqsColor || (MANY && LIT && LIST != 2)
                                ? 0
-                               : (LIST == 0 ? (LIT ? 8 : 9) : (LIST == 1 && !MANY ? 6 : 5)) * 128 / BLOCK;
+                           : LIST == 1 ? ((MANY ? 5 : 6) * 128 + BLOCK - 1) / BLOCK
+                                       : (LIST == 2 ? 5 : LIT ? 8 : 9) * 128 / BLOCK;
 
 // How the pair uniforms reach an instance.  On 16 bytes the compiler reads them
 // two pairs at a time, which the index raster gains from (100M flight 795 -> 774
