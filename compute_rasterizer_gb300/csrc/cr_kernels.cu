@@ -259,8 +259,10 @@ __device__ __forceinline__ void emit_read(const BatchedLaunch& bl, unsigned long
         ok[j] = ok[j] && !zcache_rejects(zc, zslot_pixel(pix[j]), pix[j], wb[j]);
         depth[j] = 0xFFFFFFFFu;
         if (ok[j]) {
-            const uint32_t* high = reinterpret_cast<const uint32_t*>(fb + (pix[j] - bias)) + 1;
-            asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(depth[j]) : "l"(high) : "memory");
+            // the whole word, as the atomics write it (the high half alone is no faster)
+            unsigned long long word;
+            asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(word) : "l"(fb + (pix[j] - bias)) : "memory");
+            depth[j] = (uint32_t)(word >> 32);
         }
     }
 #pragma unroll
