@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(512, 2) k_morton_keys(MortonFrame f, const uin
 // one of 40M at 10 times 13.3 ms, now 6.6; 1.2 and 6.8 with passes over all bits).
 // A run belongs to the CTA of its first key, which writes the keys that moved; the
 // neighbouring CTA, which has its last keys too, takes only their upper bits, which
-// no move changes.
+// no move changes (loads and stores are relaxed accesses, since they may meet).
 constexpr int kMaxRun = 64, kRunTile = 1024;
 __global__ void __launch_bounds__(256) k_sort_runs(unsigned long long* keys, uint32_t* idx, int64_t n, int low,
                                                    uint32_t* flag) {
@@ -438,8 +438,8 @@ __global__ void __launch_bounds__(256) k_sort_runs(unsigned long long* keys, uin
         const int cnt = (int)min((int64_t)(kRunTile + kMaxRun), n - base);  // keys from base on
         const int before = base > 0 ? 1 : 0;
         for (int k = (int)threadIdx.x - before; k < cnt; k += 256) {
-            s_key[1 + k] = keys[base + k];
-            s_idx[1 + k] = idx[base + k];
+            asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(s_key[1 + k]) : "l"(keys + base + k) : "memory");
+            asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(s_idx[1 + k]) : "l"(idx + base + k) : "memory");
         }
         __syncthreads();
         for (int i = 1 + threadIdx.x; i <= cnt; i += 256) {
@@ -453,12 +453,12 @@ __global__ void __launch_bounds__(256) k_sort_runs(unsigned long long* keys, uin
             while (last < cnt && last - first < kMaxRun && s_key[last + 1] >> low == head)
                 at += s_key[++last] < key;
             if (last - first + 1 >= kMaxRun) {  // (may go on past the copy)
-                if (i == first) *flag = 1u;
+                if (i == first) *reinterpret_cast<volatile uint32_t*>(flag) = 1u;
                 continue;
             }
             if (at == i) continue;
-            keys[base + at - 1] = key;
-            idx[base + at - 1] = s_idx[i];
+            asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(keys + base + at - 1), "l"(key) : "memory");
+            asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(idx + base + at - 1), "r"(s_idx[i]) : "memory");
         }
     }
 }
