@@ -922,18 +922,23 @@ cr_status cr_morton_sort_device(cr_ctx* ctx, uint8_t* d_rec, int64_t n, int32_t 
                                                         vals.Current(), aligned ? copy : nullptr);
         e = cudaGetLastError();
     }
-    // Radix passes over the upper 40 bits (48 above 2^26 points), 5 (6) in place of 8
-    // at 0.3 ms each for 40M points; k_sort_runs (0.2 ms) finishes the runs they leave
-    // equal.  A surface scan fills about two bits of three, so 40 bits are 2^26 cells
-    // and runs stay short; points so clustered that a run reaches kMaxRun (a far
-    // outlier stretches the header's cube, or duplicates) get the passes over all bits
-    // after all.  The sort then takes, against all bits at once with allocations of
-    // its own: 40M points 6.1-6.6 ms (6.7-6.9), 5M 0.99-1.17 (1.2), 300k 302 us (495).
-    // Up to kFullKeys points, where it would lose (80,000 points 280 us against 245,
-    // 10,000 335 against 145), all bits come first and only: 131 us at 10,000 points,
-    // 166 at 65,536 (115 and 145 by the short passes, where no run is long).
+    // Radix passes over the upper 40 bits, 5 in place of 8 at 0.3 ms each for 40M
+    // points; k_sort_runs (0.2 ms) finishes the runs they leave equal.  A surface scan
+    // fills about two bits of three, so 40 bits are 2^26 cells and runs stay short;
+    // points so clustered that a run reaches kMaxRun (a far outlier stretches the
+    // header's cube, or duplicates) get the passes over all bits after all.  The sort
+    // then takes, against all bits at once with allocations of its own: 40M points
+    // 6.1-6.6 ms (6.7-6.9), 5M 0.99-1.17 (1.2), 300k 302 us (495).  Where a clustered
+    // cloud would lose, all bits come first and only:
+    //   up to kFullKeys points (10,000 by both sorts 335 us, 80,000 280, against 145 and
+    //   245): 131 us at 10,000 points, 166 at 65,536 (115 and 145 by the short passes,
+    //   where no run is long);
+    //   above 2^26, whose cells take 48 bits, 6 passes (200M by both 37.6-38.9 ms
+    //   against 33.0-33.7, 600M 112-116 against 96-99): 29.9-30.6 and 90-92 ms; 31.2 and
+    //   93.7 where no run is long (28.7 and 86.6 by the short passes, 34.3 and 100 with
+    //   allocations of its own).
     constexpr int64_t kFullKeys = 8 * cr::kPointsPerBatch;
-    const int low = n <= kFullKeys ? 0 : n <= ((int64_t)1 << 26) ? 23 : 15;
+    const int low = n <= kFullKeys || n > ((int64_t)1 << 26) ? 0 : 23;
     if (e == cudaSuccess)
         e = cub::DeviceRadixSort::SortPairs(cub_tmp, cub_bytes, keys, vals, (int)n, low, 63, s);
     if (low > 0) {
