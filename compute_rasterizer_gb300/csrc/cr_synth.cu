@@ -525,7 +525,7 @@ __device__ __forceinline__ uint32_t quantize30(double d, double size, double inv
 
 // One batch's box and quantisation from the integer extremes, in shared memory.
 struct EncodeBox {
-    double box[9];  // min, max, 1 / size
+    double box[6], size[3], inv[3];  // min and max; max - min; 1 / size
     cr::QuantFx fx[3];
     cr::QuantQuick qq[3];
 };
@@ -534,6 +534,7 @@ struct EncodeBox {
 // The batch AABB of v = double(X) * scale + offset - boxMin
 // (LasLoaderSparse.cpp:93-105): every step rounds monotonically, so v is
 // monotone in the integer X and the box is v at the integer extremes.
+template <bool QUICK>
 __device__ __forceinline__ void encode_box(const EncodeArgs& a, int32_t mn[3], int32_t mx[3], int64_t first,
                                            int cnt, cr_batch* batches, EncodeBox& s_b) {
     __shared__ int32_t s_red[6][32];
@@ -561,9 +562,10 @@ __device__ __forceinline__ void encode_box(const EncodeArgs& a, int32_t mn[3], i
         const double b0 = a.scale[k] < 0.0 ? vhi : vlo, b1 = a.scale[k] < 0.0 ? vlo : vhi;
         s_b.box[k] = b0;
         s_b.box[3 + k] = b1;
-        s_b.box[6 + k] = 1.0 / (b1 - b0);
+        s_b.size[k] = b1 - b0;
+        s_b.inv[k] = 1.0 / (b1 - b0);
         s_b.fx[k] = cr::quant_setup(a.scale[k], a.offset[k], a.box_min[k], b0, true, b1 - b0, 30, lo, hi);
-        s_b.qq[k] = cr::quant_quick_setup(s_b.fx[k]);
+        if (QUICK) s_b.qq[k] = cr::quant_quick_setup(s_b.fx[k]);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -578,19 +580,20 @@ __device__ __forceinline__ void encode_box(const EncodeArgs& a, int32_t mn[3], i
     }
 }
 
-// One point to word `pi` of the streams, from its integer coordinates X (a
-// callable of the axis) and its color word.  Each coordinate's 30-bit cell in
-// integer arithmetic where the error bound decides it (cr_quant.h), else the
-// double chain: the same integer either way.
 // The rest of the points, out of line: it would cost the common path registers.
 __device__ __noinline__ uint32_t encode_exact(const EncodeArgs& a, const EncodeBox& s_b, int k, int32_t x) {
     uint32_t q;
     if (cr::quant_fast(s_b.fx[k], x, 1073741823u, &q)) return q;
     const double v = (double)x * a.scale[k] + a.offset[k] - a.box_min[k];
-    return quantize30(v - s_b.box[k], s_b.box[3 + k] - s_b.box[k], s_b.box[6 + k]);
+    return quantize30(v - s_b.box[k], s_b.size[k], s_b.inv[k]);
 }
 
-template <typename F>
+// One point to word `pi` of the streams, from its integer coordinates X (a
+// callable of the axis) and its color word.  Each coordinate's 30-bit cell in
+// integer arithmetic where the error bound decides it (cr_quant.h), else the
+// double chain: the same integer either way.
+// QUICK false: quant_quick's setup was left out.
+template <bool QUICK, typename F>
 __device__ __forceinline__ void encode_point(const EncodeArgs& a, const EncodeBox& s_b, F X, uint32_t color,
                                              int64_t pi, uint32_t* lo, uint32_t* md, uint32_t* hi, uint32_t* rgba) {
     uint32_t l = 0, m = 0, h = 0;
@@ -598,7 +601,9 @@ __device__ __forceinline__ void encode_point(const EncodeArgs& a, const EncodeBo
     for (int k = 0; k < 3; k++) {
         const int32_t x = X(k);
         uint32_t q;
-        if (!cr::quant_quick(s_b.qq[k], x, 1073741823u, &q)) q = encode_exact(a, s_b, k, x);
+        const bool done = QUICK ? cr::quant_quick(s_b.qq[k], x, 1073741823u, &q)
+                                : cr::quant_fast(s_b.fx[k], x, 1073741823u, &q);
+        if (!done) q = encode_exact(a, s_b, k, x);
         l |= ((q >> 20) & 1023u) << (10 * k);
         m |= ((q >> 10) & 1023u) << (10 * k);
         h |= (q & 1023u) << (10 * k);
@@ -672,14 +677,14 @@ __global__ void __launch_bounds__(S::kThreads, S::kCtas) k_encode(EncodeArgs a, 
             }
         __syncthreads();
     }
-    encode_box(a, mn, mx, first, cnt, batches, s_b);
+    encode_box<true>(a, mn, mx, first, cnt, batches, s_b);
     for (int t = ntiles - 1; t >= 0; t--) {
         if (t < ntiles - S::kStages) wait_tile<S::kStages - 1>();
         const int m = recs(t);
         for (int i = threadIdx.x; i < m; i += S::kThreads) {
             const uint8_t* r = tile(t) + i * a.bpp;
-            encode_point(a, s_b, [&](int k) { return tile_i32<EVEN>(r + 4 * k); }, encode_color<EVEN>(a, r),
-                         first + (int64_t)t * tile_recs + i, lo, md, hi, rgba);
+            encode_point<true>(a, s_b, [&](int k) { return tile_i32<EVEN>(r + 4 * k); }, encode_color<EVEN>(a, r),
+                               first + (int64_t)t * tile_recs + i, lo, md, hi, rgba);
         }
         __syncthreads();
         fetch(t - S::kStages);
@@ -698,7 +703,10 @@ cudaError_t launch_encode(const EncodeArgs& a, const uint8_t* rec, cr_batch* bat
 }
 
 // The same straight from global memory, a load per byte: records that do not start
-// on a 16-byte boundary, or too long for a tile.
+// on a 16-byte boundary, that are long (a tile fetches all of a record, this the 18
+// bytes it needs), or few.  QUICK false: without quant_quick, whose setup costs a CTA
+// more than its few points gain.
+template <bool QUICK>
 __global__ void __launch_bounds__(256) k_encode_bytes(EncodeArgs a, const uint8_t* __restrict__ rec,
                                                       cr_batch* batches, uint32_t* lo, uint32_t* md, uint32_t* hi,
                                                       uint32_t* rgba) {
@@ -712,10 +720,10 @@ __global__ void __launch_bounds__(256) k_encode_bytes(EncodeArgs a, const uint8_
             mn[k] = min(mn[k], X);
             mx[k] = max(mx[k], X);
         }
-    encode_box(a, mn, mx, first, cnt, batches, s_b);
+    encode_box<QUICK>(a, mn, mx, first, cnt, batches, s_b);
     for (int i = threadIdx.x; i < cnt; i += blockDim.x)
-        encode_point(a, s_b, [&](int k) { return get_i32(rec + (first + i) * a.bpp + 4 * k); },
-                     encode_color<false>(a, rec + (first + i) * a.bpp), first + i, lo, md, hi, rgba);
+        encode_point<QUICK>(a, s_b, [&](int k) { return get_i32(rec + (first + i) * a.bpp + 4 * k); },
+                            encode_color<false>(a, rec + (first + i) * a.bpp), first + i, lo, md, hi, rgba);
 }
 
 __host__ __device__ inline cr_vertex uniform_vertex(uint64_t seed, uint64_t i, float size) {
@@ -782,17 +790,29 @@ cr_status cr::encode_records_device(const uint8_t* d_rec, int64_t n, int32_t bpp
     a.rgb = rgb < 0 ? -1 : rgb;
     a.file_index = file_index;
     cudaStream_t s = (cudaStream_t)stream;
-    if (tile_records(bpp, EncodeMany::kBytes) == 0 || (reinterpret_cast<uintptr_t>(d_rec) & 15) != 0) {
-        k_encode_bytes<<<(unsigned)nb, 256, 0, s>>>(a, d_rec, d_batches, d_lo, d_md, d_hi, d_rgba);
+    // Where neither tiles nor the quick form pay.  us by the bytes / by tiles (before there
+    // were tiles): 1,000 points 15.5 / 18.5 (15.5), 2,000 19.1 / 19.7 (19.4), 4,500 25.6 /
+    // 23.7 (27.4); 10M points of 300 bytes 549 / 912 (710), 100k 71 / 126 (83), 6M of 200
+    // bytes 324 / 386 (380), of 140 300 / 292 (384), of 100 238 / 225 (288).
+    constexpr int64_t kFewPoints = 2048;
+    constexpr int32_t kTileMaxBpp = 140;
+    if (n <= kFewPoints) {
+        k_encode_bytes<false><<<(unsigned)nb, 256, 0, s>>>(a, d_rec, d_batches, d_lo, d_md, d_hi, d_rgba);
+        return cuda_status(cudaGetLastError());
+    }
+    if (bpp > kTileMaxBpp || (reinterpret_cast<uintptr_t>(d_rec) & 15) != 0) {
+        k_encode_bytes<true><<<(unsigned)nb, 256, 0, s>>>(a, d_rec, d_batches, d_lo, d_md, d_hi, d_rgba);
         return cuda_status(cudaGetLastError());
     }
     int device = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (e == cudaSuccess) {
-        const auto launch = nb <= sms       ? launch_encode<EncodeFew>
-                            : nb <= 2 * sms ? launch_encode<EncodeTwo>
-                                            : launch_encode<EncodeMany>;
+        // (the ring of EncodeFew holds most of a batch of 28-byte records; of 34 bytes, 600k
+        // points took 44.1 us with it, 42.1 in EncodeTwo)
+        const auto launch = nb <= sms && bpp <= 28 ? launch_encode<EncodeFew>
+                            : nb <= 2 * sms        ? launch_encode<EncodeTwo>
+                                                   : launch_encode<EncodeMany>;
         e = launch(a, d_rec, d_batches, d_lo, d_md, d_hi, d_rgba, (unsigned)nb, s);
     }
     return cuda_status(e);
