@@ -943,8 +943,12 @@ cr_status cr_morton_sort_device(cr_ctx* ctx, uint8_t* d_rec, int64_t n, int32_t 
     if (!aligned) e = cudaMemcpyAsync(copy, d_rec, (size_t)n * bpp, cudaMemcpyDeviceToDevice, s);
     if (e == cudaSuccess && !allow_shared(k_morton_keys, 2 * kTileBytes)) e = cudaErrorInvalidConfiguration;
     if (e == cudaSuccess) {
-        const int tile = tile_records(bpp, kTileBytes);  // bpp <= kGatherMaxBpp: at least 832
-        const int grid = (int)std::min<int64_t>((n + tile - 1) / tile, 2 * (int64_t)cr_ctx_num_sms(ctx));
+        // bpp <= kGatherMaxBpp: at least 832; less for few points, so that every SM has
+        // some (its FP64 unit is slow where a cube's cells put points on their borders:
+        // 10,000 points in a cube of 2^21 units 169 -> 134 us per sort)
+        const int ctas = 2 * cr_ctx_num_sms(ctx);
+        const int tile = (int)std::min<int64_t>(tile_records(bpp, kTileBytes), std::max<int64_t>((n / ctas + 16) & ~15, 128));
+        const int grid = (int)std::min<int64_t>((n + tile - 1) / tile, ctas);
         k_morton_keys<<<grid, 512, 2 * kTileBytes, s>>>(f, aligned ? d_rec : copy, n, bpp, tile, keys.Current(),
                                                         vals.Current(), aligned ? copy : nullptr);
         e = cudaGetLastError();
