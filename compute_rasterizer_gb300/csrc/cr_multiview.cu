@@ -267,7 +267,7 @@ __device__ __forceinline__ void merge_keys(int a, int b, bool ok[4], const uint3
 }
 
 // Merges the thread's 4 candidates of one view and emits what is left.  The
-// kernel is bound by instruction issue and the L1 data pipe together (76 % each,
+// kernel is bound by instruction issue and the L1 data pipe together (80 and 73 %,
 // 40M points); pairs, merges and the unit split took the frame of 200M points
 // and 64 views from 8416 to 6836 us, 40M 2292 -> 1822, one stereo pair of 20M
 // 139 -> 87.  Branching merges and emits measured 6810, but 813 against 730 us
